@@ -187,6 +187,7 @@ struct cgfd_problem {
   std::vector<Face> faces;
 
   cgfd::SrcHost src;
+  bool src_top = false;  // a source's smoothing points reach the top plane
   std::vector<int> src_shot;
   int *d_it_begin = nullptr, *d_ext_num = nullptr, *d_src_shot = nullptr;
   long long *d_ext_idx = nullptr;
@@ -332,13 +333,13 @@ struct cgfd_problem {
   // Line receivers and slices: samples of w_pre at the start of the step, after the stations
   // (io_line_keep and io_slice_nc_put follow io_recv_keep, drv_rk_curv_col.cu:199-206).
   template <typename R>
-  int enqueue_outputs(int step) {
+  int enqueue_outputs(int step, cudaStream_t st) {
     int n = 0;
     if (nline > 0) {
       cgfd::RecvPT<R> r;
       r.nsta = nline; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_line_idx8; r.w8 = d_line_w8;
       r.pre = rptr<R>(wbuf[step & 1]); r.sf = sf; r.seis = d_line_seis; r.d_it = d_it; r.d_flag = d_flag;
-      n += timed(6, [&] { return cgfd::launch_recv(r, stream); });
+      n += timed(6, [&] { return cgfd::launch_recv(r, st); });
     }
     if (slice_per_shot > 0) {
       cgfd::SliceP<R> q;
@@ -347,7 +348,7 @@ struct cgfd_problem {
       q.pre = rptr<R>(wbuf[step & 1]);
       q.nxs = nslx; q.nys = nsly; q.nzs = nslz; q.idx = d_slice_idx;
       q.ring = d_slices; q.ring_steps = slice_ring; q.per_shot = slice_per_shot; q.d_it = d_it;
-      n += timed(6, [&] { return cgfd::launch_slices(q, stream); });
+      n += timed(6, [&] { return cgfd::launch_slices(q, st); });
     }
     return n;
   }
@@ -363,7 +364,7 @@ struct cgfd_problem {
       r.pre = rptr<double>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
       n += timed(6, [&] { return cgfd::launch_recv(r, st); });
     }
-    n += enqueue_outputs<double>(step);
+    n += enqueue_outputs<double>(step, st);
     for (int s = 0; s < 4; s++) {
       const cgfd::StagePT<double> p = stage_params_t<double>(step, s);
       n += timed(s, [&] { return cgfd::launch_stage_bulk(med, p, nzc, st); });
@@ -405,7 +406,7 @@ struct cgfd_problem {
       r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
       n += timed(6, [&] { return cgfd::launch_recv(r, st); });
     }
-    n += enqueue_outputs<float>(step);
+    n += enqueue_outputs<float>(step, st);
     float *jpre = jbuf[step & 1], *jend = jbuf[(step + 1) & 1];
     const float *jcurs[4] = {jpre, jbuf[2], jbuf[3], jbuf[2]};
     float *jouts[4] = {jbuf[2], jbuf[3], jbuf[2], nullptr};
@@ -468,7 +469,7 @@ struct cgfd_problem {
       r.pre = rptr<R>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
       n += timed(6, [&] { return cgfd::launch_recv(r, st); });
     }
-    n += enqueue_outputs<R>(step);
+    n += enqueue_outputs<R>(step, st);
     for (int s = 0; s < 4; s++) {
       const cgfd::StagePT<R> p = stage_params_t<R>(step, s);
       n += timed(s, [&] {
@@ -518,18 +519,44 @@ struct cgfd_problem {
     if (fp64) return enqueue_step64(step);
     cudaStream_t st = stream;
     int n = 0;
-    if (rec.n > 0) {
-      cgfd::RecvP r;
-      r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-      r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
-      n += timed(6, [&] { return cgfd::launch_recv(r, st); });
-    }
-    n += enqueue_outputs<float>(step);
+    // Outside per-kernel timing the side stream carries, beside the bulk tiles of a stage, what they
+    // do not depend on:
+    //   every stage: the flux pass and the surface slab (latency-bound, top planes only: they
+    //     write planes of the stage outputs that no bulk tile reads or writes in this stage);
+    //   stage 0: the station, line and slice samples (they read w_pre, which stage 0 leaves alone);
+    //   stage 3: peak motion (top plane of w_end, complete after the slab unless a source reaches
+    //     that plane) and the step counter, which the stage's sources then read one ahead.
+    // On the main stream these small kernels took 17 us of every step (5% of a 100x100x60 step).
+    const bool fork = use_tma && tiles.n > 0 && !timing;
+    const bool early_peak = fork && free_top && !src_top;
+    auto sample = [&](cudaStream_t s2) {
+      int k = 0;
+      if (rec.n > 0) {
+        cgfd::RecvP r;
+        r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
+        r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+        k += timed(6, [&] { return cgfd::launch_recv(r, s2); });
+      }
+      return k + enqueue_outputs<float>(step, s2);
+    };
+    auto peak = [&](cudaStream_t s2) {
+      cgfd::PgP q;
+      q.ni = ni; q.nj = nj; q.nshot = nshot; q.sx = sx; q.sf = sf;
+      q.off_top = off0 + (long long)(nk - 1) * sz;
+      q.w_end = wbuf[(step + 1) & 1]; q.w_pre = wbuf[step & 1];
+      q.pg = d_pg; q.dis = d_dis; q.dt = dt;
+      return cgfd::launch_peak_motion(q, s2);
+    };
+    if (!fork) n += sample(st);
     if (wave16)
       n += timed(7, [&] { return cgfd::launch_wave_scale(d_amax, d_srcb, d_it, nt_total, nshot, d_wsc, st); });
     for (int s = 0; s < 4; s++) {
       cgfd::StageP p = stage_params(step, s);
-      bool surface_done = false;
+      const bool beside = fork && (free_top || s == 0 || s == 3);
+      if (beside) {
+        CK(cudaEventRecord(ev_fork, st));
+        CK(cudaStreamWaitEvent(side, ev_fork, 0));
+      }
       if (use_tma) {
         cgfd::TmaP tm;
         const int pre = step & 1, end = (step + 1) & 1;
@@ -538,34 +565,26 @@ struct cgfd_problem {
         tm.pre = map_ctr[pre];
         tm.end = map_ctr[end];
         tm.coef = map_coef;
-        // Outside per-kernel timing, the flux pass and the surface slab (latency-bound, top
-        // planes only) run on a side stream beside the bulk tiles: they write only the top
-        // planes of the stage outputs, which no bulk tile reads or writes in this stage.
-        const bool fork = free_top && tiles.n > 0 && !timing;
-        surface_done = fork;
         n += timed(s, [&] {
-          if (fork) {
-            CK(cudaEventRecord(ev_fork, st));
-            CK(cudaStreamWaitEvent(side, ev_fork, 0));
-          }
-          int k = cgfd::launch_stage_bulk_tma(med, coef_type, wave16, shape, p, tm, p.dir[2] ? tiles_dn : tiles, st);
-          if (surface_done)
-            k += cgfd::launch_timg_flux(coef_type, wave16, p, side) +
-                 cgfd::launch_stage_surface(med, coef_type, wave16, p, side);
-          if (fork) {
-            CK(cudaEventRecord(ev_join, side));
-            CK(cudaStreamWaitEvent(st, ev_join, 0));
-          }
-          return k;
+          return cgfd::launch_stage_bulk_tma(med, coef_type, wave16, shape, p, tm, p.dir[2] ? tiles_dn : tiles, st);
         });
       } else {
         n += timed(s, [&] { return cgfd::launch_stage_bulk(med, p, nzc, st); });
       }
-      if (!surface_done)
-        n += timed(4, [&] {
-          return cgfd::launch_timg_flux(coef_type, wave16, p, st) +
-                 cgfd::launch_stage_surface(med, coef_type, wave16, p, st);
-        });
+      const cudaStream_t top = beside ? side : st;
+      n += timed(4, [&] {
+        return cgfd::launch_timg_flux(coef_type, wave16, p, top) +
+               cgfd::launch_stage_surface(med, coef_type, wave16, p, top);
+      });
+      if (beside) {
+        if (s == 0) n += sample(side);
+        if (s == 3) {
+          if (early_peak) n += peak(side);
+          n += cgfd::launch_advance(d_it, side);
+        }
+        CK(cudaEventRecord(ev_join, side));
+        CK(cudaStreamWaitEvent(st, ev_join, 0));
+      }
       if (src.nsrc > 0) {
         cgfd::SrcP q;
         q.nsrc = src.nsrc; q.max_ext = src.max_ext; q.max_nt = src.max_nt;
@@ -573,20 +592,14 @@ struct cgfd_problem {
         q.ca = p.ca; q.cb = p.cb;
         q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
         q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it;
+        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it; q.it_ahead = beside && s == 3;
         q.wave16 = wave16; q.wsc = d_wsc; q.amax = d_amax;
         n += timed(5, [&] { return cgfd::launch_source(q, st); });
       }
     }
-    if (free_top) {  // drv_rk_curv_col.cu:519-527: after the last stage, before the level swap
-      cgfd::PgP q;
-      q.ni = ni; q.nj = nj; q.nshot = nshot; q.sx = sx; q.sf = sf;
-      q.off_top = off0 + (long long)(nk - 1) * sz;
-      q.w_end = wbuf[(step + 1) & 1]; q.w_pre = wbuf[step & 1];
-      q.pg = d_pg; q.dis = d_dis; q.dt = dt;
-      n += cgfd::launch_peak_motion(q, st);
-    }
-    n += cgfd::launch_advance(d_it, st);
+    // drv_rk_curv_col.cu:519-527: after the last stage, before the level swap
+    if (free_top && !early_peak) n += peak(st);
+    if (!fork) n += cgfd::launch_advance(d_it, st);
     return n;
   }
 
@@ -1216,6 +1229,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
     size_t ne = (size_t)s.nsrc * s.max_ext;
     std::vector<long long> idx(ne, p->off0);
     for (size_t e = 0; e < ne; e++) idx[e] = p->didx(s.ext_i[e], s.ext_j[e], s.ext_k[e]);
+    for (size_t e = 0; e < ne; e++) p->src_top |= s.ext_k[e] == p->nk - 1;
     p->d_it_begin = dmalloc<int>(s.nsrc, B, p->stream);
     p->d_ext_num = dmalloc<int>(s.nsrc, B, p->stream);
     p->d_ext_idx = dmalloc<long long>(ne, B, p->stream);

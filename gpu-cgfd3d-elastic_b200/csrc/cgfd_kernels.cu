@@ -433,37 +433,41 @@ __global__ void __launch_bounds__(32 * 2 * NSURF, 2) k_stage_surface(const __gri
 // -----------------------------------------------------------------------------------------
 // sources, stations, step counter
 // -----------------------------------------------------------------------------------------
+// One thread per (component, smoothing point): the kernel is a chain of dependent loads (step ->
+// time function -> weight) ended by one or two reductions, so its time is that chain's latency.
+// One thread per point with the 9 components in turn took 7.4 us per launch (343 points, one
+// source), four launches a step on the critical path of every grid; this form takes 3 us. The
+// reductions return no value except where the FP16 scale collector needs it.
 template <typename R>
 __global__ void k_source(const __grid_constant__ SrcPT<R> s) {
-  const int is = blockIdx.y;
+  const int is = blockIdx.y, c = blockIdx.z;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (is >= s.nsrc || e >= s.ext_num[is]) return;
-  const int it = *s.d_it;
-  const int ib = s.it_begin[is];
-  if (it < ib || it > ib + s.max_nt - 1) return;
-  const float *v = s.stf + (((long long)is * s.max_nt + (it - ib)) * 4 + s.stage) * 9;
-  const int shot = s.src_shot[is];
-  const long long id = s.ext_idx[(long long)is * s.max_ext + e] + (long long)shot * 9 * s.sf;
-  const R wv = s.ext_wv[(long long)is * s.max_ext + e];
-  const R wt = s.ext_wt[(long long)is * s.max_ext + e];
-  for (int c = 0; c < 9; c++) {
-    R h;
-    if (c < 3) { if (!s.force) continue; h = R(v[c]) * wv; }
-    else { if (!s.moment) continue; h = -R(v[c]) * wt; }
-    if (s.stage < 3) {
-      if constexpr (std::is_same<R, float>::value) {
-        if (s.wave16)
-          atomicAdd(reinterpret_cast<__half *>(s.tmp_out) + c * s.sf + id,
-                    __float2half_rn(s.ca * h * s.wsc[18 * shot + 9 + c]));
-        else atomicAdd(s.tmp_out + c * s.sf + id, s.ca * h);
-      } else {
-        atomicAdd(s.tmp_out + c * s.sf + id, s.ca * h);
-      }
+  if (is >= s.nsrc || (c < 3 ? !s.force : !s.moment)) return;
+  const int it = *s.d_it - s.it_ahead;
+  const int ib = s.it_begin[is], ne = s.ext_num[is], shot = s.src_shot[is];
+  if (e >= ne || it < ib || it > ib + s.max_nt - 1) return;
+  const long long q = (long long)is * s.max_ext + e;
+  const long long id = s.ext_idx[q] + ((long long)shot * 9 + c) * s.sf;
+  const R w = (c < 3 ? s.ext_wv : s.ext_wt)[q];
+  const R v = s.stf[(((long long)is * s.max_nt + (it - ib)) * 4 + s.stage) * 9 + c];
+  const R h = c < 3 ? v * w : -v * w;
+  if (s.stage < 3) {
+    if constexpr (std::is_same<R, float>::value) {
+      if (s.wave16)
+        atomicAdd(reinterpret_cast<__half *>(s.tmp_out) + id, __float2half_rn(s.ca * h * s.wsc[18 * shot + 9 + c]));
+      else atomicAdd(s.tmp_out + id, s.ca * h);
+    } else {
+      atomicAdd(s.tmp_out + id, s.ca * h);
     }
-    const R old = atomicAdd(s.end + c * s.sf + id, s.cb * h);
-    if constexpr (std::is_same<R, float>::value)
-      if (s.wave16 && s.stage == 3) atomic_max_abs(&s.amax[2 * shot + wgroup(c)], old + s.cb * h);
   }
+  if constexpr (std::is_same<R, float>::value) {
+    if (s.wave16 && s.stage == 3) {
+      const R old = atomicAdd(s.end + id, s.cb * h);
+      atomic_max_abs(&s.amax[2 * shot + wgroup(c)], old + s.cb * h);
+      return;
+    }
+  }
+  atomicAdd(s.end + id, s.cb * h);
 }
 
 template <typename R>
@@ -486,7 +490,9 @@ __global__ void k_recv(const __grid_constant__ RecvPT<R> r) {
 
 // PG_calcu_gpu (wav_t.cu:281-360) on the top physical plane, every shot: acceleration from the
 // step difference of V, displacement accumulated by the trapezoid rule in double (the
-// reference's 0.5 literal), running maxima of the components and magnitudes.
+// reference's 0.5 literal), running maxima of the components and magnitudes. Every load is issued
+// before the first store: one thread per surface point leaves too few warps to hide 15 dependent
+// load-compare-store rounds (12 us per step on 64x64 and 480x480 points alike; 4-6 us now).
 template <typename R>
 __global__ void k_peak_motion(const __grid_constant__ PgPT<R> q) {
   const long long nij = (long long)q.ni * q.nj;
@@ -498,12 +504,20 @@ __global__ void k_peak_motion(const __grid_constant__ PgPT<R> q) {
   const long long idx = (long long)shot * 9 * q.sf + q.off_top + (long long)j * q.sx + i;
   R v1[3], v0[3], a[3], d[3];
   R *dis = q.dis + (long long)shot * 3 * nij + ij;
+  float *pg = q.pg + (long long)shot * 15 * nij + ij;
+  float old[15];
+#pragma unroll
+  for (int n = 0; n < 15; n++) old[n] = pg[n * nij];
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    v1[c] = q.w_end[c * q.sf + idx];
-    v0[c] = q.w_pre[c * q.sf + idx];
+    v1[c] = __ldg(q.w_end + c * q.sf + idx);
+    v0[c] = __ldg(q.w_pre + c * q.sf + idx);
+    d[c] = dis[c * nij];
+  }
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
     a[c] = fabs((v1[c] - v0[c]) / R(q.dt));
-    d[c] = (R)((double)dis[c * nij] + 0.5 * (double)(v1[c] + v0[c]) * (double)q.dt);
+    d[c] = (R)((double)d[c] + 0.5 * (double)(v1[c] + v0[c]) * (double)q.dt);
     dis[c * nij] = d[c];
   }
   const R val[15] = {sqrt(v1[0] * v1[0] + v1[1] * v1[1] + v1[2] * v1[2]),
@@ -515,10 +529,9 @@ __global__ void k_peak_motion(const __grid_constant__ PgPT<R> q) {
                      sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]),
                      sqrt(d[0] * d[0] + d[1] * d[1]),
                      fabs(d[0]), fabs(d[1]), fabs(d[2])};
-  float *pg = q.pg + (long long)shot * 15 * nij + ij;
 #pragma unroll
   for (int n = 0; n < 15; n++)
-    if (pg[n * nij] < (float)val[n]) pg[n * nij] = (float)val[n];
+    if (old[n] < (float)val[n]) pg[n * nij] = (float)val[n];
 }
 
 template <typename R>
@@ -929,7 +942,7 @@ template <typename R>
 int launch_source(const SrcPT<R> &s, cudaStream_t st) {
   if (s.nsrc <= 0) return 0;
   dim3 block(128);
-  dim3 grid((s.max_ext + 127) / 128, s.nsrc);
+  dim3 grid((s.max_ext + 127) / 128, s.nsrc, 9);
   k_source<R><<<grid, block, 0, st>>>(s);
   return 1;
 }

@@ -32,6 +32,7 @@ struct SrcPT {
   R *end;
   long long sf;
   const int *d_it;
+  int it_ahead;                // steps the counter is already ahead of the step being run (0 or 1)
   int wave16;                  // FP16 stage levels: tmp_out holds scaled __half
   const float *wsc;            // [nshot][18] scale / inverse scale of this step (wave16)
   unsigned int *amax;          // [nshot][2] max |w_end| per group, collected at stage 3 (wave16)
