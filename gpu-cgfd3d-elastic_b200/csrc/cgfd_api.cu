@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -968,6 +969,7 @@ std::vector<float> source_bounds(const cgfd_problem *p) {
 }
 
 void make_tiles(cgfd_problem *p);
+int default_chunk(const cgfd_problem *p);
 void make_maps(cgfd_problem *p);
 void make_ac_maps(cgfd_problem *p);
 float *noalloc_scratch(int device);
@@ -1069,14 +1071,9 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
   // device layout
   layout(p->ni, p->nj, p->nk, p->sx, p->sz, p->sf, p->off0);
   // default tiling (cgfd_set_tile_shape / cgfd_set_zchunk / the autotuner refine it): 32x4
-  // tiles at three blocks per SM for iso media, the shape-0 tiles otherwise, and z chunks of
-  // about 12 planes (with strip-ordered tile lists a chunk's 3-plane prologue comes from L2, and
-  // short chunks keep the resident blocks on neighbouring planes)
+  // tiles at three blocks per SM for iso media, the shape-0 tiles otherwise, z chunks by
+  // default_chunk once the PML faces are known
   p->shape = p->med == cgfd::MED_ISO ? 1 : 0;
-  {
-    int chunks = std::max(1, (p->nbulk + 11) / 12);
-    p->nzc = (p->nbulk + chunks - 1) / chunks;
-  }
 
   size_t &B = p->bytes;
   // levels 0-1 (w_pre / w_end) FP32; 2-3 (RK stage inputs) FP32 or FP16
@@ -1285,6 +1282,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
     CK(cudaMemcpy(p->d_w8, p->rec.w8.data(), p->rec.w8.size() * sizeof(float), cudaMemcpyHostToDevice));
     CK(cudaMemset(p->d_seis, 0, sizeof(float) * p->rec.n * 9 * p->nt_total * nshot));
   }
+  p->nzc = default_chunk(p);
   make_tiles(p);
   if (p->free_top) {
     const size_t nij = (size_t)p->ni * p->nj * nshot;
@@ -1361,6 +1359,70 @@ void make_ac_maps(cgfd_problem *p) {
            p->ncoef);
 }
 
+// z ranges of the tile list: [0, nbulk) cut at the z-face boundaries of the CFS-PML, each part split
+// into chunks of at most about nzc planes.
+std::vector<std::pair<int, int>> z_ranges(const cgfd_problem *p, int nzc) {
+  std::vector<int> cuts = {0, p->nbulk};
+  for (const auto &f : p->faces)
+    if (f.h.axis == 2)
+      for (int c : {f.h.lo[2], f.h.hi[2] + 1})
+        if (c > 0 && c < p->nbulk) cuts.push_back(c);
+  std::sort(cuts.begin(), cuts.end());
+  cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
+  std::vector<std::pair<int, int>> zr;
+  for (size_t s = 0; s + 1 < cuts.size(); s++) {
+    const int len = cuts[s + 1] - cuts[s], nch = std::max(1, (len + nzc - 1) / nzc);
+    for (int c = 0; c < nch; c++) zr.emplace_back(cuts[s] + len * c / nch, cuts[s] + len * (c + 1) / nch);
+  }
+  return zr;
+}
+
+// Default z chunk of the bulk (or acoustic) stage kernel. A grid of several resident sets of blocks
+// takes chunks of about 12 planes: a chunk's 3-plane prologue comes from L2, and short chunks keep
+// the resident blocks on neighbouring planes. A grid with fewer blocks than kFew resident sets at 12
+// planes is bound by the time its last set takes, so it takes the chunk length c that minimises
+// ceil(blocks / resident) (longest chunk + 3): sets of blocks, each as long as its longest block with
+// its prologue. us per step, 12 planes against the rule's choice: 64x64x64 235 against 122 (4
+// planes), 100x100x60 312 against 283 (5 planes); 5 shots of 141x118x77, 6.5 sets, 1780 at 12 planes
+// and 1785-1830 at 4-8.
+int default_chunk(const cgfd_problem *p) {
+  constexpr int kFew = 3, kPrologue = 3;
+  if (p->nbulk < 1) return 1;
+  int nsm = 148;
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
+  const bool tiled = p->use_tma;
+  const int ty = tiled ? cgfd::tma_tile_y(p->med, p->shape) : cgfd::TY;
+  const int per_sm = tiled ? cgfd::tma_resident(p->med, p->coef_type, p->wave16, p->shape)
+                           : p->fp64 ? 1 : p->med == cgfd::MED_AC ? 3 : 2;
+  const long long resident = (long long)nsm * per_sm;
+  const long long columns = (long long)((p->ni + cgfd::TX - 1) / cgfd::TX) * ((p->nj + ty - 1) / ty) * p->nshot;
+  auto even = [&](int c) {  // the chunk length of nbulk planes in equal chunks of at most c
+    const int n = (p->nbulk + c - 1) / c;
+    return (p->nbulk + n - 1) / n;
+  };
+  auto chunks = [&](int c, int &longest) {
+    if (!tiled) {
+      longest = std::min(c, p->nbulk);
+      return (p->nbulk + c - 1) / c;
+    }
+    const auto zr = z_ranges(p, c);
+    longest = 0;
+    for (const auto &z : zr) longest = std::max(longest, z.second - z.first);
+    return (int)zr.size();
+  };
+  int longest = 0;
+  const int usual = even(12);
+  if (columns * chunks(usual, longest) >= kFew * resident) return usual;
+  int best = usual;
+  long long best_cost = LLONG_MAX;
+  for (int c = 12; c >= 3; c--) {
+    const long long blocks = columns * chunks(c, longest);
+    const long long cost = (blocks + resident - 1) / resident * (longest + kPrologue);
+    if (cost < best_cost) { best_cost = cost; best = c; }
+  }
+  return best;
+}
+
 // Tile lists of the TMA bulk kernel: 32 x TY columns, split along z into chunks of about
 // nzc planes that never straddle a z-face boundary of the CFS-PML (so planes above the
 // bottom absorbing layer run as tiles without face code); a tile that any PML face box meets
@@ -1373,21 +1435,10 @@ void make_ac_maps(cgfd_problem *p) {
 // (tiles), downwards for forward ones (tiles_dn).
 void make_tiles(cgfd_problem *p) {
   if (p->med == cgfd::MED_AC) return;  // no TMA kernel for acoustic media
-  const int ty = cgfd::tma_tile_y(p->med, p->shape), nbulk = p->nbulk;
+  const int ty = cgfd::tma_tile_y(p->med, p->shape);
   const int nbx = (p->ni + cgfd::TX - 1) / cgfd::TX, nby = (p->nj + ty - 1) / ty;
   if (nbx > cgfd::kTileBxMask + 1) throw cgfd::Error(CGFD_ERR_INVALID, "grid too wide for the bulk tile list");
-  std::vector<int> cuts = {0, nbulk};
-  for (const auto &f : p->faces)
-    if (f.h.axis == 2)
-      for (int c : {f.h.lo[2], f.h.hi[2] + 1})
-        if (c > 0 && c < nbulk) cuts.push_back(c);
-  std::sort(cuts.begin(), cuts.end());
-  cuts.erase(std::unique(cuts.begin(), cuts.end()), cuts.end());
-  std::vector<std::pair<int, int>> zr;
-  for (size_t s = 0; s + 1 < cuts.size(); s++) {
-    const int len = cuts[s + 1] - cuts[s], nch = std::max(1, (len + p->nzc - 1) / p->nzc);
-    for (int c = 0; c < nch; c++) zr.emplace_back(cuts[s] + len * c / nch, cuts[s] + len * (c + 1) / nch);
-  }
+  const auto zr = z_ranges(p, p->nzc);
   int nsm = 148;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
   const int group = std::max(1, std::min(p->shot_group, p->nshot));

@@ -26,6 +26,25 @@ int tma_blocks_per_sm(int med, int shape) {
   return shape ? TileShape<MED_ANISO, 1>::MINB : TileShape<MED_ANISO, 0>::MINB;
 }
 
+template <int MED, int SH, typename TC, typename TW>
+static int resident_of() {
+  using S = BulkSmem<MED, TileShape<MED, SH>::TYT, TC, TW, TileShape<MED, SH>::MINB>;
+  const int by_smem = 228 * 1024 / (S::BYTES + 1024), by_regs = 65536 / (128 * TX * TileShape<MED, SH>::TYT);
+  return by_smem < by_regs ? by_smem : by_regs;
+}
+
+template <int MED, int SH>
+static int resident_med(int coef_type, int wave16) {
+  if (wave16) return resident_of<MED, SH, uint16_t, __half>();
+  return coef_type == COEF_F32 ? resident_of<MED, SH, float, float>() : resident_of<MED, SH, uint16_t, float>();
+}
+
+int tma_resident(int med, int coef_type, int wave16, int shape) {
+  if (med == MED_ISO) return shape ? resident_med<MED_ISO, 1>(coef_type, wave16) : resident_med<MED_ISO, 0>(coef_type, wave16);
+  if (med == MED_VTI) return shape ? resident_med<MED_VTI, 1>(coef_type, wave16) : resident_med<MED_VTI, 0>(coef_type, wave16);
+  return shape ? resident_med<MED_ANISO, 1>(coef_type, wave16) : resident_med<MED_ANISO, 0>(coef_type, wave16);
+}
+
 cudaError_t tma_prepare(int med, int coef_type, int wave16, int shape) {
   if (med == MED_ISO) return prepare_bulk_tma_med<MED_ISO>(coef_type, wave16, shape);
   if (med == MED_VTI) return prepare_bulk_tma_med<MED_VTI>(coef_type, wave16, shape);

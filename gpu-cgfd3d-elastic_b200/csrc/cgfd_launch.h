@@ -153,6 +153,9 @@ int launch_timg_flux64(const StagePT<double> &p, cudaStream_t st);
 // shape: tile shape index (0 default, 1 the alternative; cgfd_bulk_tma.cuh TileShape)
 int tma_tile_y(int med, int shape);
 int tma_blocks_per_sm(int med, int shape);  // resident blocks per SM the tile shape is built for
+// blocks an SM holds of the tile shape with that coefficient and wave storage (shared memory,
+// 128 registers per thread)
+int tma_resident(int med, int coef_type, int wave16, int shape);
 cudaError_t tma_prepare(int med, int coef_type, int wave16, int shape);
 // Tile list of the TMA bulk kernel (device array, one int4 per block in launch order:
 // bx + kTilePml if a CFS-PML face meets the tile + (shot << 16), by, first and end z plane).
