@@ -29,6 +29,7 @@
 #include "cgfd_dev.cuh"
 #include "cgfd_launch.h"
 #include "cgfd_setup.h"
+#include "cgfd_stager.h"
 #include "cgfd_tma.cuh"
 
 namespace {
@@ -37,12 +38,8 @@ thread_local std::string g_err;
 
 void set_err(const std::string &m) { g_err = m; }
 
-#define CK(call)                                                                                 \
-  do {                                                                                           \
-    cudaError_t e_ = (call);                                                                     \
-    if (e_ != cudaSuccess)                                                                       \
-      throw cgfd::Error(CGFD_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));      \
-  } while (0)
+#define CK CGFD_CK
+using cgfd::PinnedStager;
 
 // 8 pairs of forward/backward flags (fd_t.cu:184-194), direction = (flag + stage) % 2
 const int kPairFlags[8][3] = {{0, 0, 0}, {1, 1, 0}, {1, 1, 1}, {0, 0, 1},
@@ -671,88 +668,6 @@ int guarded(Fn fn) {
     return CGFD_ERR_INVALID;
   }
 }
-
-// Host -> device copies of the caller's model arrays (pageable memory) through two pinned
-// chunks: host threads fill one chunk while the copy engine drains the other, so the upload
-// runs at the slower of a parallel host memcpy and the host link instead of the driver's
-// serial pageable path. One stager per device, allocated on first use and kept for the life
-// of the process (2 x 64 MiB of pinned host memory): allocating and freeing pinned memory per
-// problem would synchronise the device under the serving loop's concurrent problems. Users
-// hold its lock for a whole upload; each chunk is refilled only after the copy out of it
-// has completed (per-chunk events), so no device-wide synchronisation is involved.
-class PinnedStager {
- public:
-  static constexpr size_t kChunk = size_t(64) << 20;
-  // fields below this size go through the plain pageable copy
-  static constexpr size_t kMinBytes = size_t(16) << 20;
-
-  static PinnedStager &for_device(int device) {
-    static std::mutex mu;
-    static std::vector<PinnedStager *> all;
-    std::lock_guard<std::mutex> lk(mu);
-    if ((int)all.size() <= device) all.resize(device + 1, nullptr);
-    if (!all[device]) all[device] = new PinnedStager();  // device is current
-    return *all[device];
-  }
-  std::mutex &mutex() { return mu_; }
-
-  // device -> caller's (pageable) host memory, the reverse pipeline: the copy engine fills one
-  // chunk while host threads empty the other
-  void copy_out(void *dst, const void *src, size_t n, cudaStream_t st) {
-    const size_t nch = (n + kChunk - 1) / kChunk;
-    auto issue = [&](size_t c) {
-      const size_t o = c * kChunk, m = std::min(kChunk, n - o);
-      CK(cudaEventSynchronize(done_[c & 1]));
-      CK(cudaMemcpyAsync(buf_[c & 1], static_cast<const char *>(src) + o, m, cudaMemcpyDeviceToHost, st));
-      CK(cudaEventRecord(done_[c & 1], st));
-    };
-    if (nch > 0) issue(0);
-    for (size_t c = 0; c < nch; c++) {
-      if (c + 1 < nch) issue(c + 1);
-      CK(cudaEventSynchronize(done_[c & 1]));
-      const size_t o = c * kChunk, m = std::min(kChunk, n - o);
-      char *out = static_cast<char *>(dst) + o;
-      const long long pieces = (long long)((m + kPiece - 1) / kPiece);
-#pragma omp parallel for schedule(static)
-      for (long long q = 0; q < pieces; q++) {
-        const size_t a = (size_t)q * kPiece;
-        std::memcpy(out + a, buf_[c & 1] + a, std::min(kPiece, m - a));
-      }
-    }
-    next_ = (int)(nch & 1);
-  }
-
-  void copy(void *dst, const void *src, size_t n, cudaStream_t st) {
-    for (size_t o = 0; o < n; o += kChunk) {
-      const size_t m = std::min(kChunk, n - o);
-      const int b = next_;
-      next_ ^= 1;
-      CK(cudaEventSynchronize(done_[b]));  // the previous copy out of this chunk has finished
-      const char *in = static_cast<const char *>(src) + o;
-      const long long pieces = (long long)((m + kPiece - 1) / kPiece);
-#pragma omp parallel for schedule(static)
-      for (long long q = 0; q < pieces; q++) {
-        const size_t a = (size_t)q * kPiece;
-        std::memcpy(buf_[b] + a, in + a, std::min(kPiece, m - a));
-      }
-      CK(cudaMemcpyAsync(static_cast<char *>(dst) + o, buf_[b], m, cudaMemcpyHostToDevice, st));
-      CK(cudaEventRecord(done_[b], st));
-    }
-  }
-
- private:
-  PinnedStager() {
-    for (int b = 0; b < 2; b++) {
-      CK(cudaHostAlloc(reinterpret_cast<void **>(&buf_[b]), kChunk, cudaHostAllocPortable));
-      CK(cudaEventCreateWithFlags(&done_[b], cudaEventDisableTiming));
-    }
-  }
-  static constexpr size_t kPiece = size_t(1) << 20;
-  std::mutex mu_;
-  char *buf_[2] = {nullptr, nullptr};
-  cudaEvent_t done_[2] = {nullptr, nullptr};
-  int next_ = 0;
-};
 
 // One model field (reference layout) into its device array, through stage_buf. ps: the
 // device's pinned stager, its lock held by the caller (nullptr: plain pageable copy).
@@ -1683,9 +1598,10 @@ int cgfd_get_wavefield_shot(cgfd_problem *p, int shot, float *out) {
   return guarded([&] {
     CK(cudaSetDevice(p->device));
     cgfd::RefGrid g(p->ni, p->nj, p->nk);
+    const size_t field = g.siz_icmp * sizeof(float);
     size_t acc = 0;
     float *tmp = dmalloc<float>(g.siz_icmp, acc, p->stream);
-    for (int c = 0; c < 9; c++) {
+    auto repack = [&](int c) {
       const size_t off = ((size_t)shot * 9 + c) * p->sf;
       if (p->fp64)
         cgfd::launch_repack_out(p->rptr<double>(p->wbuf[p->it & 1], off), tmp, p->ni, p->nj, p->nk, p->sx, p->sz,
@@ -1693,9 +1609,23 @@ int cgfd_get_wavefield_shot(cgfd_problem *p, int shot, float *out) {
       else
         cgfd::launch_repack_out(p->rptr<float>(p->wbuf[p->it & 1], off), tmp, p->ni, p->nj, p->nk, p->sx, p->sz,
                                 p->off0, p->stream);
-      CK(cudaMemcpyAsync(out + (size_t)c * g.siz_icmp, tmp, g.siz_icmp * sizeof(float), cudaMemcpyDeviceToHost, p->stream));
+    };
+    try {
+      if (field >= PinnedStager::kMinOut) {
+        PinnedStager &ps = PinnedStager::for_device(p->device);
+        std::lock_guard<std::mutex> lk(ps.mutex());
+        ps.copy_out(out, tmp, field, 9, p->stream, repack);
+      } else {
+        for (int c = 0; c < 9; c++) {
+          repack(c);
+          CK(cudaMemcpyAsync(out + (size_t)c * g.siz_icmp, tmp, field, cudaMemcpyDeviceToHost, p->stream));
+        }
+      }
+      CK(cudaStreamSynchronize(p->stream));
+    } catch (...) {
+      dfree(tmp, p->stream);
+      throw;
     }
-    CK(cudaStreamSynchronize(p->stream));
     dfree(tmp, p->stream);
   });
 }

@@ -35,3 +35,17 @@ def test_default_chunk_changes_no_result(medium, grid):
     p = small_problem(medium, *grid, nsteps=4, npml=3, nsrc=1)
     (a,), (b,) = _two_steps(p), _two_steps(p, setup=lambda s: s.set_zchunk(12))
     np.testing.assert_array_equal(a, b)
+
+
+# a field below the staged copy's least size, one of a single chunk, one of a chunk and a remainder
+@pytest.mark.parametrize("grid", [(40, 36, 30), (120, 100, 70), (300, 280, 210)])
+def test_wavefield_readback_equals_box(grid):
+    p = small_problem("iso", *grid, nsteps=2, npml=0, nsrc=0, sta_grid=None)
+    sim = Simulation(p)
+    rng = np.random.default_rng(1)
+    w = np.zeros((9,) + tuple(n + 6 for n in grid[::-1]), np.float32)
+    w[:, 3:-3, 3:-3, 3:-3] = rng.standard_normal((9,) + grid[::-1], dtype=np.float32)
+    sim.set_wavefield(w)
+    out = sim.wavefield()
+    np.testing.assert_array_equal(out, w)
+    np.testing.assert_array_equal(out[:, 3:-3, 3:-3, 3:-3], sim.wavefield_box((0, 0, 0), grid))
