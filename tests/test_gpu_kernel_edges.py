@@ -8,7 +8,8 @@ equal to double rounding, so their read-back floats differ by one unit in the la
 import numpy as np
 import pytest
 
-from cgfd_b200 import Simulation
+from cgfd_b200 import Simulation, media_layer_gpu, CGFD_MEDIA_ARI, CGFD_MEDIA_HAR
+from cgfd_b200.formats import LayerModel
 from helpers import small_problem, random_wavefield
 
 pytestmark = pytest.mark.gpu
@@ -49,3 +50,49 @@ def test_wavefield_readback_equals_box(grid):
     out = sim.wavefield()
     np.testing.assert_array_equal(out, w)
     np.testing.assert_array_equal(out[:, 3:-3, 3:-3, 3:-3], sim.wavefield_box((0, 0, 0), grid))
+
+
+@pytest.mark.parametrize("method", [CGFD_MEDIA_HAR, CGFD_MEDIA_ARI])
+@pytest.mark.parametrize("dims", [(8, 8, 8), (19, 11, 14)])
+def test_layer_averages_at_mixed_points(method, dims):
+    """Flat layers on a Cartesian grid: the 9^3 sub-points of a mixed half-grid cell lie on 9
+    elevations, those within 1 m of an interface take the mean of both layers (the reference's
+    integer test). A float sum of 729 terms is within 729 x 2^-24 = 4.4e-5 of the exact one."""
+    ni, nj, nk = dims
+    dh = 100.0
+    coord = np.zeros((3, nk + 6, nj + 6, ni + 6), np.float32)
+    coord[0] = (np.arange(-3, ni + 3) * dh)[None, None, :]
+    coord[1] = (np.arange(-3, nj + 3) * dh)[None, :, None]
+    coord[2] = (np.arange(-3, nk + 3) * dh - (nk - 1) * dh)[:, None, None]
+    tops = [float(coord[2].max()) + 500.0, -233.0, -512.0]
+    par = {"vp": [4000.0, 5500.0, 6500.0], "vs": [2300.0, 3200.0, 3750.0], "rho": [2500.0, 2700.0, 2900.0]}
+    shape = (3, 4, 5)
+    f = {"elevation": np.array(tops, np.float32)[:, None, None] * np.ones(shape, np.float32)}
+    for n, v in par.items():
+        f[n] = np.array(v, np.float32)[:, None, None] * np.ones(shape, np.float32)
+        f[n + "_grad"] = np.zeros(shape, np.float32)
+        f[n + "_pow"] = np.ones(shape, np.float32)
+    m = LayerModel(float(coord[0].min()) - 50, float(coord[1].min()) - 50, 1000.0, 1000.0, **f)
+    got = media_layer_gpu(coord, m, method)
+
+    def values(z):  # (rho, lambda, mu) at elevation z
+        n = max(q for q in range(3) if tops[q] >= z)
+        layers = [n - 1, n] if n > 0 and int(tops[n] - z) == 0 else [n]
+        rho, vp, vs = (np.mean([par[k][q] for q in layers]) for k in ("rho", "vp", "vs"))
+        return np.array([rho, rho * vp * vp - 2 * rho * vs * vs, rho * vs * vs])
+
+    mixed = 0
+    for k in range(1, nk + 5):
+        z = float(coord[2, k, 0, 0])
+        lo, hi = z - dh / 2, z + dh / 2
+        if max(q for q in range(3) if tops[q] >= lo) == max(q for q in range(3) if tops[q] >= hi):
+            want = values(z)
+        else:
+            mixed += 1
+            v = np.array([values(lo + (hi - lo) / 8 * s) for s in range(9)])
+            want = v.mean(0)
+            if method == CGFD_MEDIA_HAR:
+                mu = 1 / np.mean(1 / v[:, 2])
+                want = np.array([want[0], 1 / np.mean(1 / (v[:, 1] + 2 / 3 * v[:, 2])) - 2 / 3 * mu, mu])
+        np.testing.assert_allclose(got[:, k, 1:-1, 1:-1], want[:, None, None] * np.ones((3, nj + 4, ni + 4)), rtol=5e-5)
+    assert mixed >= 2
