@@ -44,28 +44,27 @@ __global__ void k_ac_image(R *cur, R *end_ghost, int ni, int nj, int nk, long lo
 
 // CFS-PML work of one face for one acoustic cell (sv_curv_col_ac_iso_gpu.cu:647-802): the 1-D
 // terms of this axis rhs_d; h += (B-1) rhs_d - B aux; aux' = D rhs_d - A aux; RK combine of the
-// 4 auxiliary variables (component stride n, shot stride 9 n as for the elastic faces).
+// 4 auxiliary variables (components 0-3 of the elastic faces' layout).
 template <typename R>
 __device__ __forceinline__ void ac_pml_face(const StagePT<R> &p, const FacePT<R> &f, int i, int j, int k, int shot,
                                             R slw, R kappa, const R m[3], const R dv[3], R dp, R hc[kAcF]) {
   const int ab = f.axis == 0 ? i - f.lo[0] : (f.axis == 1 ? j - f.lo[1] : k - f.lo[2]);
   const R cA = __ldg(f.A + ab), cB = __ldg(f.B + ab), cD = __ldg(f.D + ab);
   const R cB1 = cB - R(1);
-  const long long ia =
-      (long long)shot * 9 * f.n + ((long long)(k - f.lo[2]) * f.ny + (j - f.lo[1])) * f.nx + (i - f.lo[0]);
+  AuxPoint<kAcF, false, R> aux;
+  aux.load(f, p.stage, i, j, k, shot);
   R rhs[kAcF];
   rhs[0] = -slw * (m[0] * dp);
   rhs[1] = -slw * (m[1] * dp);
   rhs[2] = -slw * (m[2] * dp);
   rhs[3] = -kappa * (m[0] * dv[0] + m[1] * dv[1] + m[2] * dv[2]);
-  R aux[kAcF], arhs[kAcF];
+  R arhs[kAcF];
 #pragma unroll
   for (int c = 0; c < kAcF; c++) {
-    aux[c] = f.aux_cur[c * f.n + ia];
-    hc[c] += cB1 * rhs[c] - cB * aux[c];
-    arhs[c] = cD * rhs[c] - cA * aux[c];
+    hc[c] += cB1 * rhs[c] - cB * aux.cur[c];
+    arhs[c] = cD * rhs[c] - cA * aux.cur[c];
   }
-  rk_store<kAcF>(p.stage, p.ca, p.cb, f.n, ia, aux, arhs, f.aux_pre, f.aux_tmp, f.aux_end);
+  aux.store(f, p.stage, p.ca, p.cb, arhs);
 }
 
 template <typename R>

@@ -179,10 +179,11 @@ struct cgfd_problem {
   struct Face {
     cgfd::PmlFaceHost h;
     float *A = nullptr, *B = nullptr, *D = nullptr;
-    float *aux = nullptr;  // [3][9][n]
-    long long n = 0;
+    float *aux = nullptr;  // [nshot][blocks][3 levels][9][32] (cgfd_dev.cuh)
+    long long plane = 0, blocks = 0;  // 32-point blocks per z plane of the box, per shot
   };
   std::vector<Face> faces;
+  int aux_flip = 0;  // the auxiliaries' pre level is (step + aux_flip) & 1 (cgfd_set_step)
 
   cgfd::SrcHost src;
   bool src_top = false;  // a source's smoothing points reach the top plane
@@ -315,15 +316,14 @@ struct cgfd_problem {
       for (int b = 0; b < 3; b++) { o.lo[b] = f.h.lo[b]; o.hi[b] = f.h.hi[b]; }
       o.nx = f.h.hi[0] - f.h.lo[0] + 1;
       o.ny = f.h.hi[1] - f.h.lo[1] + 1;
-      o.n = f.n;
+      o.plane = f.plane;
+      o.shot = f.blocks;
       o.A = rptr<R>(f.A); o.B = rptr<R>(f.B); o.D = rptr<R>(f.D);
-      const size_t L = (size_t)nshot * 9 * f.n;
-      R *apre = rptr<R>(f.aux, (size_t)(step & 1) * L), *aend = rptr<R>(f.aux, (size_t)((step + 1) & 1) * L);
-      R *atmp = rptr<R>(f.aux, (size_t)2 * L);
-      o.aux_cur = stage == 0 ? apre : atmp;
-      o.aux_pre = apre;
-      o.aux_tmp = atmp;
-      o.aux_end = aend;
+      o.aux = rptr<R>(f.aux);
+      o.pre = ((step + aux_flip) & 1) * cgfd::kAuxLevel;
+      o.end = cgfd::kAuxLevel - o.pre;
+      o.tmp = 2 * cgfd::kAuxLevel;
+      o.cur = stage == 0 ? o.pre : o.tmp;
     }
     return p;
   }
@@ -791,6 +791,11 @@ void layout(int ni, int nj, int nk, long long &sx, long long &sz, long long &sf,
   off0 = 3 * sz + 3 * sx + cgfd::GX;
 }
 
+// 32-point blocks per z plane of a CFS-PML face box (the auxiliaries' layout, cgfd_dev.cuh)
+long long aux_plane(const cgfd::PmlFaceHost &h) {
+  return ((long long)(h.hi[0] - h.lo[0] + 1) * (h.hi[1] - h.lo[1] + 1) + 31) / 32;
+}
+
 // Device bytes build() holds once done (*resident) and at its high-water mark (*peak), from
 // the description alone (host work only: PML, source and station setup).
 void problem_bytes(const cgfd_problem_desc *d, int nshot, const cgfd_source_desc *shots, size_t *resident,
@@ -823,8 +828,7 @@ void problem_bytes(const cgfd_problem_desc *d, int nshot, const cgfd_source_desc
     for (int s = 0; s < 2; s++) {
       if (!fh[a][s].enable) continue;
       const cgfd::PmlFaceHost &h = fh[a][s];
-      const size_t n = (size_t)(h.hi[0] - h.lo[0] + 1) * (h.hi[1] - h.lo[1] + 1) * (h.hi[2] - h.lo[2] + 1);
-      r += 3 * h.A.size() * F + (size_t)3 * 9 * n * nshot * F;
+      r += 3 * h.A.size() * F + (size_t)aux_plane(h) * (h.hi[2] - h.lo[2] + 1) * cgfd::kAuxBlock * nshot * F;
     }
   size_t nsrc = 0, max_ext = 0, max_nt = 0;
   for (int sh = 0; sh < (shots ? nshot : 1); sh++) {
@@ -1077,14 +1081,16 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
       if (!fh[a][s].enable) continue;
       cgfd_problem::Face f;
       f.h = fh[a][s];
-      f.n = (long long)(f.h.hi[0] - f.h.lo[0] + 1) * (f.h.hi[1] - f.h.lo[1] + 1) * (f.h.hi[2] - f.h.lo[2] + 1);
+      f.plane = aux_plane(f.h);
+      f.blocks = f.plane * (f.h.hi[2] - f.h.lo[2] + 1);
+      const size_t naux = (size_t)nshot * f.blocks * cgfd::kAuxBlock;
       size_t N1 = f.h.A.size();
       f.A = dalloc_real(p, N1, B); f.B = dalloc_real(p, N1, B); f.D = dalloc_real(p, N1, B);
       upload_real(p, f.A, f.h.A);
       upload_real(p, f.B, f.h.B);
       upload_real(p, f.D, f.h.D);
-      f.aux = dalloc_real(p, (size_t)3 * 9 * f.n * nshot, B);
-      CK(cudaMemset(f.aux, 0, E * 3 * 9 * f.n * nshot));
+      f.aux = dalloc_real(p, naux, B);
+      CK(cudaMemset(f.aux, 0, E * naux));
       p->faces.push_back(f);
     }
   // sources: one set per shot, concatenated (each source knows its shot)
@@ -1411,7 +1417,7 @@ void reset_state(cgfd_problem *p) {
   const size_t E = p->esz;
   const size_t lev_bytes[4] = {E, E, p->wave16 ? 2u : E, p->wave16 ? 2u : E};
   for (int l = 0; l < 4; l++) CK(cudaMemsetAsync(p->wbuf[l], 0, lev_bytes[l] * 9 * p->sf * p->nshot, p->stream));
-  for (auto &f : p->faces) CK(cudaMemsetAsync(f.aux, 0, E * 3 * 9 * f.n * p->nshot, p->stream));
+  for (auto &f : p->faces) CK(cudaMemsetAsync(f.aux, 0, E * p->nshot * f.blocks * cgfd::kAuxBlock, p->stream));
   for (auto *jb : p->jbuf)
     if (jb) CK(cudaMemsetAsync(jb, 0, sizeof(float) * 6 * p->nmax * p->sf, p->stream));
   if (p->rec.n > 0)
@@ -1555,13 +1561,7 @@ int cgfd_set_step(cgfd_problem *p, int it) {
       std::swap(p->wbuf[0], p->wbuf[1]);
       std::swap(p->map_halo[0], p->map_halo[1]);
       std::swap(p->map_ctr[0], p->map_ctr[1]);
-      for (auto &f : p->faces) {
-        size_t n = (size_t)9 * f.n * p->nshot;
-        void *l0 = p->rvoid(f.aux, 0), *l1 = p->rvoid(f.aux, n), *l2 = p->rvoid(f.aux, 2 * n);
-        CK(cudaMemcpyAsync(l2, l0, n * p->esz, cudaMemcpyDeviceToDevice, p->stream));
-        CK(cudaMemcpyAsync(l0, l1, n * p->esz, cudaMemcpyDeviceToDevice, p->stream));
-        CK(cudaMemcpyAsync(l1, l2, n * p->esz, cudaMemcpyDeviceToDevice, p->stream));
-      }
+      p->aux_flip ^= 1;
       for (int s = 0; s < 8; s++)
         if (p->graph_ok[s]) { cudaGraphExecDestroy(p->graph[s]); p->graph_ok[s] = false; }
     }

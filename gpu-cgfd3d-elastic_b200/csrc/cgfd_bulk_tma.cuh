@@ -67,6 +67,10 @@ struct BulkSmem {
   static constexpr int OFF_CPE = NW * WAVE_SLOT;
   static constexpr int OFF_BAR = OFF_CPE + 2 * CPE_SLOT;
   static constexpr int BYTES = OFF_BAR + 8 * 8;
+  // resident blocks the registers are budgeted for: a fourth 32x4 block of iso tiles (57 KB each)
+  // fits beside three at 128 registers per thread, and is worth 3-5% over three at 168
+  static constexpr int BOUND = MED == MED_ISO && MINB == 3 && 4 * (BYTES + 1024) <= 228 * 1024 ? 4 : MINB;
+  static constexpr bool ONE_ROUND = sizeof(real_of<TC>) == 4 && BOUND * CELLS * 168 <= 65536;
   static_assert(NW + 2 <= 8, "mbarrier area");
   static_assert(COEF_BYTES % 128 == 0, "w_pre/w_end boxes must stay 128-byte aligned");
   static_assert(MINB == 1 || MINB * (BYTES + 1024) <= 228 * 1024, "MINB blocks must fit one SM's shared memory");
@@ -149,14 +153,16 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
     issue_cpe(0);
   }
 
-  // PML faces that intersect this block (uniform)
-  unsigned fmask = 0;
+  // PML faces that intersect this block (uniform), and those this thread's column lies in: z chunks
+  // are cut at the z faces, so a column's faces are the same at every plane of the tile
+  unsigned fmask = 0, tmask = 0;
   for (int fi = 0; PML && fi < p.nface; fi++) {
     const FaceP &f = p.face[fi];
     const bool xo = f.lo[0] <= bx * TX + TX - 1 && f.hi[0] >= bx * TX;
     const bool yo = f.lo[1] <= by * TYT + TYT - 1 && f.hi[1] >= by * TYT;
     const bool zo = f.lo[2] <= ke - 1 && f.hi[2] >= kb;
     if (xo && yo && zo) fmask |= 1u << fi;
+    if (act && in_face(f, i, j, k0)) tmask |= 1u << fi;
   }
 
   // register queue of the planes behind, in march order: q[f][n] = plane k + (n - 3) * SD
@@ -247,22 +253,22 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
         // (x1 x2 y1 y2 z1), as the reference applies its face kernels after the inner one;
         // the face axis' derivatives are recomputed here, when the accumulators above are
         // dead, to keep the face code's registers free
-        if (fmask)
-          for (int fi = 0; fi < p.nface; fi++) {
-            const FaceP &fc = p.face[fi];
-            if (!(fmask >> fi & 1) || !in_face(fc, i, j, k)) continue;
-            float d[9];
-            if (fc.axis == 0) {
-              deriv_x(d);
-              pml_face<MED>(p, fc, i, j, k, md, slw, mt[0], d, d + 3, nullptr, nullptr, h, shot);
-            } else if (fc.axis == 1) {
-              deriv_y(d);
-              pml_face<MED>(p, fc, i, j, k, md, slw, mt[1], d, d + 3, nullptr, nullptr, h, shot);
-            } else {
-              deriv_z(d);
-              pml_face<MED>(p, fc, i, j, k, md, slw, mt[2], d, d + 3, nullptr, nullptr, h, shot);
-            }
+        for (unsigned left = fmask; left; left &= left - 1) {
+          const int fi = __ffs(left) - 1;
+          if (!(tmask >> fi & 1)) continue;
+          const FaceP &fc = p.face[fi];
+          float d[9];
+          if (fc.axis == 0) {
+            deriv_x(d);
+            pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[0], d, d + 3, nullptr, nullptr, h, shot);
+          } else if (fc.axis == 1) {
+            deriv_y(d);
+            pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[1], d, d + 3, nullptr, nullptr, h, shot);
+          } else {
+            deriv_z(d);
+            pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[2], d, d + 3, nullptr, nullptr, h, shot);
           }
+        }
       }
       // RK combine (wav_update / wav_update_end)
       const long long id = didx(p, i, j, k);
@@ -330,7 +336,7 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
 // others its compiled-out form. Both kinds in one launch keep a tile's x-y neighbours, PML or
 // not, resident beside it, so that the halo lines they share are read from DRAM once.
 template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP>
-__global__ void __launch_bounds__(TX *TYT, MINB)
+__global__ void __launch_bounds__(TX *TYT, BulkSmem<MED, TYT, TC, typename WavePolicy<WP>::TW, MINB>::BOUND)
     k_stage_bulk_tma(const __grid_constant__ StageP p, const __grid_constant__ TmaP tm,
                      const int4 *__restrict__ tiles) {
   const int4 tl = __ldg(tiles + blockIdx.x);

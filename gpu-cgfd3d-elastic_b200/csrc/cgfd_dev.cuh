@@ -52,21 +52,24 @@ template <> struct MedInfo<MED_AC>    { static constexpr int NCOEF = 11; };
 // precision, every production mode) or double (the FP64 build, CGFD_PREC_FP64).
 
 // One CFS-PML face (bdry_t.cu:85-257): box [lo,hi] in physical indices, 1-D A/B/D along the
-// face normal, and the 9-component auxiliary variables (component stride n) at the levels
-// this stage reads and writes.
+// face normal, and the auxiliary variables. The box's points are numbered x fastest, y, then z with
+// every z plane rounded up to a whole number of 32-point blocks; a block holds its 3 levels x 9
+// components x 32 points together. So one pointer per point reaches all 27 values a stage needs at
+// constant offsets, and they lie in 3.4 KB of DRAM instead of in 27 places a component or level
+// apart (kAuxBlock values per block).
+constexpr int kAuxComp = 32, kAuxLevel = 9 * kAuxComp, kAuxBlock = 3 * kAuxLevel;
 template <typename R>
 struct FacePT {
   int enable;
   int axis;           // 0 x, 1 y, 2 z
   int lo[3], hi[3];   // inclusive box, physical 0-based indices
   int nx, ny;         // box extents along x, y
-  long long n;        // points in the box
+  long long plane;    // blocks per z plane of the box
+  long long shot;     // blocks per shot
   const R *A, *B, *D;
-  // each level holds nshot x 9 components (shot stride 9 n)
-  const R *aux_cur;   // level read by the RHS (pre at stage 0, tmp otherwise)
-  const R *aux_pre;   // pre level (stages 1-2)
-  R *aux_tmp;         // tmp level written at stages 0-2 (== aux_cur at stages 1-2)
-  R *aux_end;         // end level
+  R *aux;
+  int cur, pre, tmp, end;  // offsets of the levels this stage reads (cur: pre at stage 0, tmp otherwise;
+                           // pre: stages 1-2) and writes (tmp: stages 0-2; end)
 };
 using FaceP = FacePT<float>;
 
@@ -306,6 +309,62 @@ constexpr int kErrWaveNonfinite = 4;     // the RK combine produced a NaN/Inf so
 __device__ __forceinline__ bool nonfinite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 __device__ __forceinline__ bool nonfinite(double v) { return !(fabs(v) <= 1.7976931348623157e308); }
 
+// This point's auxiliaries: component c of level offset l (cur, pre, tmp, end) at [l + c * kAuxComp].
+template <typename R>
+__device__ __forceinline__ R *face_aux(const FacePT<R> &f, int i, int j, int k, int shot) {
+  const int q = (j - f.lo[1]) * f.nx + (i - f.lo[0]);
+  const long long b = shot * f.shot + (k - f.lo[2]) * f.plane + (q >> 5);
+  return f.aux + b * kAuxBlock + (q & 31);
+}
+
+// The N auxiliaries of one point and their RK combine. ONE_ROUND: what the combine reads is loaded
+// together with the stage input, one round trip to memory instead of two, for kernels with the
+// registers to hold 3 N values across the right-hand side (168 per thread: 21-Cij tiles 1345 -> 1244 us
+// per step on 203x187x121, against 1316 in two rounds); at 128 registers it spills and loses more
+// than it gains (iso tiles on 480x480x240: 10.0 ms per step before, 9.74 in two rounds, 11.1 in one).
+template <int N, bool ONE_ROUND, typename R>
+struct AuxPoint {
+  R *a;
+  R cur[N], pre[N], end[N];
+  __device__ __forceinline__ void load(const FacePT<R> &f, int stage, int i, int j, int k, int shot) {
+    a = face_aux(f, i, j, k, shot);
+#pragma unroll
+    for (int c = 0; c < N; c++) cur[c] = a[f.cur + c * kAuxComp];
+    if (ONE_ROUND) {
+      if (stage >= 1) load_end(f);
+      if (stage == 1 || stage == 2) load_pre(f);
+    }
+  }
+  __device__ __forceinline__ void load_end(const FacePT<R> &f) {
+#pragma unroll
+    for (int c = 0; c < N; c++) end[c] = a[f.end + c * kAuxComp];
+  }
+  __device__ __forceinline__ void load_pre(const FacePT<R> &f) {
+#pragma unroll
+    for (int c = 0; c < N; c++) pre[c] = a[f.pre + c * kAuxComp];
+  }
+  __device__ __forceinline__ void store(const FacePT<R> &f, int stage, R ca, R cb, const R rhs[N]) {
+    if (stage == 0) {
+#pragma unroll
+      for (int c = 0; c < N; c++) {
+        a[f.tmp + c * kAuxComp] = cur[c] + ca * rhs[c];
+        a[f.end + c * kAuxComp] = cur[c] + cb * rhs[c];
+      }
+    } else if (stage < 3) {
+      if (!ONE_ROUND) { load_pre(f); load_end(f); }
+#pragma unroll
+      for (int c = 0; c < N; c++) {
+        a[f.tmp + c * kAuxComp] = pre[c] + ca * rhs[c];
+        a[f.end + c * kAuxComp] = end[c] + cb * rhs[c];
+      }
+    } else {
+      if (!ONE_ROUND) load_end(f);
+#pragma unroll
+      for (int c = 0; c < N; c++) a[f.end + c * kAuxComp] = end[c] + cb * rhs[c];
+    }
+  }
+};
+
 // RK combine of N values at one point (wav_update / wav_update_end, wav_t.cu:362-378): the 9
 // elastic components, or the 4 acoustic ones (Vx Vy Vz P).
 // cur_c: the stage input at the point (== pre at stage 0). err (may be null): at stage 3,
@@ -354,15 +413,16 @@ __device__ __forceinline__ void rk_store(int stage, R ca, R cb, long long comp_s
 //   followed by the RK combine of the auxiliary variables.
 template <typename T> struct nondeduced { using type = T; };  // keeps nullptr arguments out of deduction
 
-template <int MED, typename R>
+template <int MED, bool ONE_ROUND = false, typename R>
 __device__ __forceinline__ void pml_face(const StagePT<R> &p, const FacePT<R> &f, int i, int j, int k,
                                          const Medium<MED, R> &md, R slw, const R m[3],
                                          const R dv[3], const R dt[6], const typename nondeduced<R>::type *surf_mat,
                                          const typename nondeduced<R>::type *zeta, R hc[9], int shot = 0) {
-  int ab = f.axis == 0 ? i - f.lo[0] : (f.axis == 1 ? j - f.lo[1] : k - f.lo[2]);
+  AuxPoint<9, ONE_ROUND, R> aux;
+  aux.load(f, p.stage, i, j, k, shot);
+  const int ab = f.axis == 0 ? i - f.lo[0] : (f.axis == 1 ? j - f.lo[1] : k - f.lo[2]);
   R cA = __ldg(f.A + ab), cB = __ldg(f.B + ab), cD = __ldg(f.D + ab);
   R cB1 = cB - R(1);
-  long long ia = (long long)shot * 9 * f.n + ((long long)(k - f.lo[2]) * f.ny + (j - f.lo[1])) * f.nx + (i - f.lo[0]);
   R rhs[9];
   momentum_axis(m, dt, rhs);
   rhs[0] *= slw; rhs[1] *= slw; rhs[2] *= slw;
@@ -374,12 +434,11 @@ __device__ __forceinline__ void pml_face(const StagePT<R> &p, const FacePT<R> &f
       for (int xj = 0; xj < 3; xj++) Ga[vi][xj] = m[xj] * dv[vi];
     md.hooke(Ga, rhs + 3);
   }
-  R aux[9], arhs[9];
+  R arhs[9];
 #pragma unroll
   for (int c = 0; c < 9; c++) {
-    aux[c] = f.aux_cur[c * f.n + ia];
-    hc[c] += cB1 * rhs[c] - cB * aux[c];
-    arhs[c] = cD * rhs[c] - cA * aux[c];
+    hc[c] += cB1 * rhs[c] - cB * aux.cur[c];
+    arhs[c] = cD * rhs[c] - cA * aux.cur[c];
   }
   if (surf_mat) {
     // dzV converted from this axis' derivative (sv_curv_col_el_iso_gpu.cu:855-915)
@@ -398,7 +457,7 @@ __device__ __forceinline__ void pml_face(const StagePT<R> &p, const FacePT<R> &f
       arhs[3 + c] += cD * hs[c];
     }
   }
-  rk_store(p.stage, p.ca, p.cb, f.n, ia, aux, arhs, f.aux_pre, f.aux_tmp, f.aux_end);
+  aux.store(f, p.stage, p.ca, p.cb, arhs);
 }
 
 template <typename R>
