@@ -233,7 +233,10 @@ __global__ void __launch_bounds__(TX *TY, AcTile<R>::MINB)
         R hc[kAcF] = {R(0), R(0), R(0), R(0)};
         for (int fi = 0; fi < p.nface; fi++) {
           const FacePT<R> &fc = p.face[fi];
-          if (in_face(fc, i, j, k)) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, m[fc.axis], dv[fc.axis], dp[fc.axis], hc);
+          if (!in_face(fc, i, j, k)) continue;
+          if (fc.axis == 0) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, m[0], dv[0], dp[0], hc);
+          else if (fc.axis == 1) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, m[1], dv[1], dp[1], hc);
+          else ac_pml_face(p, fc, i, j, k, shot, slw, kappa, m[2], dv[2], dp[2], hc);
         }
 #pragma unroll
         for (int c = 0; c < kAcF; c++) h[c] += hc[c];
@@ -455,8 +458,12 @@ __global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
         float hc[kAcF] = {0.f, 0.f, 0.f, 0.f};
         for (int fi = 0; fi < p.nface; fi++) {
           const FaceP &fc = p.face[fi];
-          if ((fmask >> fi & 1) && in_face(fc, i, j, k))
-            ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[fc.axis], dv[fc.axis], dp[fc.axis], hc);
+          if (!(fmask >> fi & 1) || !in_face(fc, i, j, k)) continue;
+          // (an index into the register arrays by fc.axis would put them in local memory for every
+          // cell, PML or not)
+          if (fc.axis == 0) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[0], dv[0], dp[0], hc);
+          else if (fc.axis == 1) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[1], dv[1], dp[1], hc);
+          else ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[2], dv[2], dp[2], hc);
         }
 #pragma unroll
         for (int c = 0; c < kAcF; c++) h[c] += hc[c];

@@ -219,16 +219,16 @@ __device__ __forceinline__ void ld5(int dir, const WaveIn<TW> &cur, int f, long 
 // J (grad xi_a . T) terms sv_curv_col_el_gpu.cu:53-217 differentiates. Computed once per point
 // here instead of once per stencil use in the surface slab.
 template <typename TC, int WP>
-__global__ void __launch_bounds__(256) k_timg_flux(const __grid_constant__ StagePT<real_of<TC>> p) {
+__global__ void __launch_bounds__(128) k_timg_flux(const __grid_constant__ StagePT<real_of<TC>> p) {
   using R = real_of<TC>;
   using TW = typename std::conditional<WP == 2, __half, R>::type;
   const int nxe = p.ni + 6, nye = p.nj + 6;
   const long long plane = (long long)nxe * nye, per_shot = 9 * kFluxPlanes * plane;
-  const long long total = plane * kFluxPlanes * p.nshot;
   const CoefView<TC> cv(p);
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-    const int ii = (int)(t % nxe), jj = (int)((t / nxe) % nye);
-    const int pl = (int)((t / plane) % kFluxPlanes), shot = (int)(t / (plane * kFluxPlanes));
+  const int ii = blockIdx.x * blockDim.x + threadIdx.x, jj = blockIdx.y * blockDim.y + threadIdx.y;
+  if (ii >= nxe || jj >= nye) return;
+  for (int z = blockIdx.z; z < kFluxPlanes * p.nshot; z += gridDim.z) {
+    const int pl = z % kFluxPlanes, shot = z / kFluxPlanes;
     const int k = p.nk - kFluxPlanes + pl;
     const long long q = didx(p, ii - 3, jj - 3, k);
     const WaveIn<TW> cur{reinterpret_cast<const TW *>(p.cur) + (long long)shot * 9 * p.sf, p.sf,
@@ -276,38 +276,49 @@ __global__ void __launch_bounds__(32 * 2 * NSURF, 2) k_stage_surface(const __gri
     Medium<MED, R> md;
     md.load([&](int c) { return cv(c, id); });
 
-    // normal derivatives of all 9 fields along the 3 axes
-    R dv[3][3], dtt[3][6];
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
+    // On the planes of the traction image the momentum comes from the fluxes: the stress derivatives
+    // (90 of a cell's 135 stencil loads) are needed there in CFS-PML faces only, which take the 9
+    // derivatives of their own axis again.
+    auto axis_derivs = [&](int a, int f0, R *d) {  // fields f0 .. 8 along axis a
 #pragma unroll
       for (int f = 0; f < 9; f++) {
+        if (f < f0) continue;
         R v[5];
         ld5(DIR[a], cur, f, id, offs[a], v);
-        R d = drp5r(DIR[a], v[0], v[1], v[2], v[3], v[4]);
-        if (f < 3) dv[a][f] = d; else dtt[a][f - 3] = d;
+        d[f] = drp5r(DIR[a], v[0], v[1], v[2], v[3], v[4]);
       }
-    }
+    };
+    R dv[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+      for (int f = 0; f < 3; f++) {
+        R v[5];
+        ld5(DIR[a], cur, f, id, offs[a], v);
+        dv[a][f] = drp5r(DIR[a], v[0], v[1], v[2], v[3], v[4]);
+      }
+    const bool image = p.free_top && k >= nk2 - (DZ ? 3 : 1);
     R hc[9];
 #pragma unroll
     for (int c = 0; c < 9; c++) hc[c] = R(0);
 
     // momentum: normal form, or the traction image near the free surface
     R h[9];
-    {
+    if (!image) {
       R mom[3] = {R(0), R(0), R(0)};
 #pragma unroll
       for (int a = 0; a < 3; a++) {
-        R mm[3];
-        momentum_axis(m[a], dtt[a], mm);
+        R d[9], mm[3];
+        axis_derivs(a, 3, d);
+        momentum_axis(m[a], d + 3, mm);
         mom[0] += mm[0]; mom[1] += mm[1]; mom[2] += mm[2];
       }
       h[0] = slw * mom[0]; h[1] = slw * mom[1]; h[2] = slw * mom[2];
     }
     constexpr int dzr = DZ;
     if (p.free_top) {
-      constexpr int idx_last = dzr ? 3 : 1, idx_first = dzr ? -1 : -3;
-      if (k >= nk2 - idx_last) {
+      constexpr int idx_first = dzr ? -1 : -3;
+      if (image) {
         // sv_curv_col_el_gpu.cu:53-217, on the fluxes k_timg_flux computed for this stage
         const int n_free = nk2 - k - idx_first;
         const R jc = __ldg(p.jac + id);
@@ -376,11 +387,21 @@ __global__ void __launch_bounds__(32 * 2 * NSURF, 2) k_stage_surface(const __gri
     // CFS-PML faces, with the free-surface terms on x/y faces at the top layer
     for (int fi = 0; fi < p.nface; fi++) {
       const FacePT<R> &fc = p.face[fi];
-      if (!(i >= fc.lo[0] && i <= fc.hi[0] && j >= fc.lo[1] && j <= fc.hi[1] && k >= fc.lo[2] && k <= fc.hi[2])) continue;
-      const int a = fc.axis;
+      if (!in_face(fc, i, j, k)) continue;
       const R *smat = nullptr;
-      if (p.free_top && a < 2 && k == nk2) smat = (a == 0 ? p.matx : p.maty) + ((long long)j * p.ni + i) * 9;
-      pml_face<MED>(p, fc, i, j, k, md, slw, m[a], dv[a], dtt[a], smat, m[2], hc, shot);
+      R d[9];
+      if (fc.axis == 0) {
+        if (p.free_top && k == nk2) smat = p.matx + ((long long)j * p.ni + i) * 9;
+        axis_derivs(0, 0, d);
+        pml_face<MED>(p, fc, i, j, k, md, slw, m[0], d, d + 3, smat, m[2], hc, shot);
+      } else if (fc.axis == 1) {
+        if (p.free_top && k == nk2) smat = p.maty + ((long long)j * p.ni + i) * 9;
+        axis_derivs(1, 0, d);
+        pml_face<MED>(p, fc, i, j, k, md, slw, m[1], d, d + 3, smat, m[2], hc, shot);
+      } else {
+        axis_derivs(2, 0, d);
+        pml_face<MED>(p, fc, i, j, k, md, slw, m[2], d, d + 3, nullptr, m[2], hc, shot);
+      }
     }
 #pragma unroll
     for (int c = 0; c < 9; c++) h[c] += hc[c];
@@ -712,9 +733,8 @@ static void launch_surface_tc(int med, const StagePT<real_of<TC>> &p, dim3 grid,
 
 template <typename TC, int WP>
 static void launch_flux_tc(const StagePT<real_of<TC>> &p, cudaStream_t st) {
-  const long long total = (long long)(p.ni + 6) * (p.nj + 6) * kFluxPlanes * p.nshot;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148 * 8);
-  k_timg_flux<TC, WP><<<blocks, 256, 0, st>>>(p);
+  const dim3 block(32, 4), grid((p.ni + 6 + 31) / 32, (p.nj + 6 + 3) / 4, std::min(kFluxPlanes * p.nshot, 65535));
+  k_timg_flux<TC, WP><<<grid, block, 0, st>>>(p);
 }
 
 int launch_timg_flux(int coef_type, int wave16, const StageP &p, cudaStream_t st) {
