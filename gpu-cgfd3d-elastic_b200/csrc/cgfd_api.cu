@@ -149,6 +149,7 @@ struct cgfd_problem {
   // memory variables [nmax][6][sf] per level (same roles as wbuf), the anelastic weights
   // [2 nmax][sf] (Ylam, then Ymu), the stage right-hand side [9][sf], the surface frame [nj][ni][9]
   int vis = 0, nmax = 0;
+  bool vis_tma = false;  // the bulk planes run the TMA kernel's visco-elastic form
   float wl[10] = {};
   float *jbuf[4] = {nullptr, nullptr, nullptr, nullptr};
   float *d_y = nullptr, *d_rhs = nullptr, *d_matD = nullptr;
@@ -392,30 +393,32 @@ struct cgfd_problem {
   }
 
   // One time step of a visco-elastic problem (drv_rk_curv_col.cu:193-541 with
-  // sv_curv_col_vis_iso_onestage): per stage the iso kernels write the right-hand side (bulk
-  // planes, then the traction-image fluxes and the surface slab), the attenuation pass combines it
-  // with the memory variables, then the sources; after the last stage the surface stress fix.
+  // sv_curv_col_vis_iso_onestage). Per stage the bulk planes run in one kernel (right-hand side,
+  // attenuation, RK combine); on the side stream, beside it, the surface slab runs in its
+  // right-hand-side mode followed by the attenuation pass of its planes. The direct-load form (more
+  // mechanisms than the fused kernel is built for, or cgfd_set_bulk_variant 0) writes the right-hand
+  // side of every plane and runs the attenuation pass over all of them. Then the sources; after the
+  // last stage the surface stress fix.
   int enqueue_step_vis(int step) {
     cudaStream_t st = stream;
     int n = 0;
-    if (rec.n > 0) {
-      cgfd::RecvPT<float> r;
-      r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-      r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
-      n += timed(6, [&] { return cgfd::launch_recv(r, st); });
-    }
-    n += enqueue_outputs<float>(step, st);
+    const bool fork = vis_tma && tiles.n > 0 && !timing;
+    auto sample = [&](cudaStream_t s2) {
+      int k = 0;
+      if (rec.n > 0) {
+        cgfd::RecvPT<float> r;
+        r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
+        r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+        k += timed(6, [&] { return cgfd::launch_recv(r, s2); });
+      }
+      return k + enqueue_outputs<float>(step, s2);
+    };
+    if (!fork) n += sample(st);
     float *jpre = jbuf[step & 1], *jend = jbuf[(step + 1) & 1];
     const float *jcurs[4] = {jpre, jbuf[2], jbuf[3], jbuf[2]};
     float *jouts[4] = {jbuf[2], jbuf[3], jbuf[2], nullptr};
     for (int s = 0; s < 4; s++) {
       cgfd::StagePT<float> p = stage_params_t<float>(step, s);
-      p.rhs = d_rhs;
-      n += timed(s, [&] { return cgfd::launch_stage_bulk(cgfd::MED_ISO, p, nzc, st); });
-      if (free_top)
-        n += timed(4, [&] {
-          return cgfd::launch_timg_flux(coef_type, 0, p, st) + cgfd::launch_stage_surface(cgfd::MED_ISO, coef_type, 0, p, st);
-        });
       cgfd::VisP v;
       memset(&v, 0, sizeof(v));
       v.ni = ni; v.nj = nj; v.nk = nk; v.nmax = nmax; v.stage = s;
@@ -425,7 +428,35 @@ struct cgfd_problem {
       v.coef = coef; v.y = d_y;
       for (int m = 0; m < nmax; m++) v.wl[m] = wl[m];
       v.ca = p.ca; v.cb = p.cb; v.err = d_flag;
-      n += timed(s, [&] { return cgfd::launch_vis_atten(v, st); });
+      const bool beside = fork && (free_top || s == 0 || s == 3);
+      if (beside) {
+        CK(cudaEventRecord(ev_fork, st));
+        CK(cudaStreamWaitEvent(side, ev_fork, 0));
+      }
+      if (vis_tma) {
+        cgfd::TmaP tm;
+        const int curs[4] = {step & 1, 2, 3, 2};
+        tm.cur = map_halo[curs[s]];
+        tm.pre = map_ctr[step & 1];
+        tm.end = map_ctr[(step + 1) & 1];
+        tm.coef = map_coef;
+        n += timed(s, [&] { return cgfd::launch_stage_bulk_vis(p, tm, v, p.dir[2] ? tiles_dn : tiles, st); });
+      }
+      p.rhs = d_rhs;
+      if (!vis_tma) n += timed(s, [&] { return cgfd::launch_stage_bulk(cgfd::MED_ISO, p, nzc, st); });
+      const cudaStream_t top = beside ? side : st;
+      if (free_top)
+        n += timed(4, [&] {
+          return cgfd::launch_timg_flux(coef_type, 0, p, top) + cgfd::launch_stage_surface(cgfd::MED_ISO, coef_type, 0, p, top);
+        });
+      v.k0 = vis_tma ? nbulk : 0;
+      n += timed(s, [&] { return cgfd::launch_vis_atten(v, top); });
+      if (beside) {
+        if (s == 0) n += sample(side);
+        if (s == 3) n += cgfd::launch_advance(d_it, side);
+        CK(cudaEventRecord(ev_join, side));
+        CK(cudaStreamWaitEvent(st, ev_join, 0));
+      }
       if (src.nsrc > 0) {
         cgfd::SrcPT<float> q;
         memset(&q, 0, sizeof(q));
@@ -434,7 +465,7 @@ struct cgfd_problem {
         q.ca = p.ca; q.cb = p.cb;
         q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
         q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it;
+        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it; q.it_ahead = beside && s == 3;
         n += timed(5, [&] { return cgfd::launch_source(q, st); });
       }
     }
@@ -450,7 +481,7 @@ struct cgfd_problem {
       q.pg = d_pg; q.dis = d_dis; q.dt = dt;
       n += cgfd::launch_peak_motion(q, st);
     }
-    n += cgfd::launch_advance(d_it, st);
+    if (!fork) n += cgfd::launch_advance(d_it, st);
     return n;
   }
 
@@ -962,7 +993,8 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
   p->wave16 = d->precision == CGFD_PREC_FP16_WAVE ? 1 : 0;
   p->fp64 = d->precision == CGFD_PREC_FP64 ? 1 : 0;
   p->esz = p->fp64 ? sizeof(double) : sizeof(float);
-  if (p->fp64 || p->vis) p->use_tma = false;  // the FP64 build and visco-elastic media run the direct-load bulk kernel
+  if (p->fp64 || p->vis) p->use_tma = false;  // the FP64 build runs the direct-load bulk kernel, visco-elastic media their own
+  p->vis_tma = p->vis && p->nmax <= cgfd::vis_bulk_max_mechanisms();
   p->device = d->device;
   CK(cudaSetDevice(p->device));
   keep_pool_memory(p->device);
@@ -1047,7 +1079,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
   if (p->coef_type != cgfd::COEF_F32) to_16bit_coefficients(p);
 
   // TMA tensor maps of the four wavefield levels and of the coefficients
-  if (p->use_tma) make_maps(p);
+  if (p->use_tma || p->vis_tma) make_maps(p);
   if (p->ac_tma) make_ac_maps(p);
   // free surface of elastic media: velocity-gradient conversion and traction-image fluxes
   if (p->free_top && p->med != cgfd::MED_AC) {
@@ -1261,7 +1293,8 @@ void make_maps(cgfd_problem *p) {
                : p->coef_type == cgfd::COEF_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                  : CU_TENSOR_MAP_DATA_TYPE_UINT16,
                2);
-    CK(cgfd::tma_prepare(p->med, p->coef_type, p->wave16, p->shape));
+    if (p->vis_tma) CK(cgfd::tma_prepare_vis(p->nmax));
+    else CK(cgfd::tma_prepare(p->med, p->coef_type, p->wave16, p->shape));
   }
 }
 
@@ -2089,6 +2122,7 @@ int cgfd_set_bulk_variant(cgfd_problem *p, int tma) {
     return CGFD_ERR_UNSUPPORTED;
   }
   p->use_tma = tma != 0;
+  p->vis_tma = false;  // visco-elastic media come here with 0 only
   for (int s = 0; s < 8; s++)
     if (p->graph_ok[s]) { cudaGraphExecDestroy(p->graph[s]); p->graph_ok[s] = false; }
   return CGFD_OK;

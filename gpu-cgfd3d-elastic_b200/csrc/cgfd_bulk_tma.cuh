@@ -22,6 +22,7 @@
 #include "cgfd_dev.cuh"
 #include "cgfd_launch.h"
 #include "cgfd_tma.cuh"
+#include "cgfd_visco.cuh"
 
 namespace cgfd {
 
@@ -86,8 +87,9 @@ struct CoefTile {
 
 // One tile (a block) of the stage; PML false: the tile meets no CFS-PML face and the face code
 // is compiled out.
-template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP, bool PML>
-__device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const int4 tl) {
+// VIS: the visco-elastic form with that many mechanisms (0: elastic; vp is then unused).
+template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP, bool PML, int VIS = 0>
+__device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const int4 tl, const VisP *vp = nullptr) {
   using TW = typename WavePolicy<WP>::TW;
   using TT = typename WavePolicy<WP>::TT;
   using S = BulkSmem<MED, TYT, TC, TW, MINB>;
@@ -270,8 +272,9 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
           }
         }
       }
-      // RK combine (wav_update / wav_update_end)
       const long long id = didx(p, i, j, k);
+      if constexpr (VIS > 0) vis_atten<VIS>(*vp, stage, id, md.lam, md.mu, h);
+      // RK combine (wav_update / wav_update_end)
       const float *PR = reinterpret_cast<const float *>(cpe + cs * S::CPE_SLOT + S::COEF_BYTES) + cell;
       const float *EN = reinterpret_cast<const float *>(cpe + cs * S::CPE_SLOT + S::OFF_END) + cell;
       const float *prg = p.pre + woff + id;  // w_pre in HBM when it is not staged

@@ -64,6 +64,7 @@ int launch_peak_motion(const PgPT<R> &q, cudaStream_t st);
 // right-hand side `rhs`, then the RK combine of the 9 wave fields and the 6 nmax memory variables.
 struct VisP {
   int ni, nj, nk, nmax, stage;
+  int k0;                             // first plane of the pass (planes [k0, nk))
   long long sx, sz, sf, off0;
   const float *rhs;                   // [9][sf] elastic right-hand side (no sources)
   const float *cur, *pre;             // wave levels: stage input, w_pre
@@ -167,6 +168,13 @@ struct BulkTiles {
 };
 int launch_stage_bulk_tma(int med, int coef_type, int wave16, int shape, const StageP &p, const TmaP &tm,
                           const BulkTiles &t, cudaStream_t st);
+// The visco-elastic form of the bulk kernel: the iso stage with the attenuation of the point and the
+// RK combine of the memory variables (v) between the right-hand side and the combine (32x4 tiles), for
+// up to vis_bulk_max_mechanisms() mechanisms (media with more run the direct-load kernel and the
+// separate attenuation pass).
+int vis_bulk_max_mechanisms();
+cudaError_t tma_prepare_vis(int nmax);
+int launch_stage_bulk_vis(const StageP &p, const TmaP &tm, const VisP &v, const BulkTiles &t, cudaStream_t st);
 // FP16 stage levels: per-step scale from the last step's max |w| and the step's source bound
 int launch_wave_scale(unsigned int *amax, const float *srcb, const int *d_it, int nt_total, int nshot, float *wsc,
                       cudaStream_t st);

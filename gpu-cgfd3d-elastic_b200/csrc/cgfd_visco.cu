@@ -16,6 +16,7 @@
 
 #include "cgfd_dev.cuh"
 #include "cgfd_launch.h"
+#include "cgfd_visco.cuh"
 
 namespace cgfd {
 
@@ -26,7 +27,7 @@ template <int NM>
 __global__ void __launch_bounds__(128) k_vis_atten(const __grid_constant__ VisP q) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= q.ni) return;
-  const int j = blockIdx.y, k = blockIdx.z;
+  const int j = blockIdx.y, k = q.k0 + blockIdx.z;
   const long long sf = q.sf;
   {
     const long long id = q.off0 + (long long)k * q.sz + (long long)j * q.sx + i;
@@ -35,50 +36,7 @@ __global__ void __launch_bounds__(128) k_vis_atten(const __grid_constant__ VisP 
     for (int f = 0; f < 9; f++) h[f] = q.rhs[f * sf + id];
     const float lam = __ldg(q.coef + (long long)CF_MED * sf + id);
     const float mu = __ldg(q.coef + (long long)(CF_MED + 1) * sf + id);
-    // strain rate from the stress rate (isotropic compliance); the diagonal in double, as the
-    // reference's double literals make it
-    const float tr = (h[3] + h[4] + h[5]) / (3.f * lam + 2.f * mu);
-    float ev[6];
-    ev[0] = (float)(((2.0 * h[3] - h[4] - h[5]) / (double)(2.f * mu) + tr) / 3.0);
-    ev[1] = (float)(((2.0 * h[4] - h[3] - h[5]) / (double)(2.f * mu) + tr) / 3.0);
-    ev[2] = (float)(((2.0 * h[5] - h[3] - h[4]) / (double)(2.f * mu) + tr) / 3.0);
-    ev[3] = (float)((double)(h[6] / mu) * 0.5);
-    ev[4] = (float)((double)(h[7] / mu) * 0.5);
-    ev[5] = (float)((double)(h[8] / mu) * 0.5);
-    float sl = 0.f, sm[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int m = 0; m < NM; m++) {
-      const float ylam = __ldg(q.y + (long long)m * sf + id);
-      const float ymu = __ldg(q.y + (long long)(NM + m) * sf + id);
-      float jc[6], hj[6];
-#pragma unroll
-      for (int c = 0; c < 6; c++) jc[c] = q.jcur[(long long)(6 * m + c) * sf + id];
-#pragma unroll
-      for (int c = 0; c < 6; c++) hj[c] = q.wl[m] * (ev[c] - jc[c]);
-      sl += ylam * (jc[0] + jc[1] + jc[2]);
-#pragma unroll
-      for (int c = 0; c < 6; c++) sm[c] += ymu * jc[c];
-      // RK combine of the memory variables
-#pragma unroll
-      for (int c = 0; c < 6; c++) {
-        const long long o = (long long)(6 * m + c) * sf + id;
-        if (q.stage == 0) {
-          q.jtmp[o] = jc[c] + q.ca * hj[c];
-          q.jend[o] = jc[c] + q.cb * hj[c];
-        } else if (q.stage < 3) {
-          q.jtmp[o] = q.jpre[o] + q.ca * hj[c];
-          q.jend[o] = q.jend[o] + q.cb * hj[c];
-        } else {
-          q.jend[o] = q.jend[o] + q.cb * hj[c];
-        }
-      }
-    }
-    const float ls = lam * sl;
-    const double mu2 = 2.0 * (double)mu;
-#pragma unroll
-    for (int c = 0; c < 3; c++) h[3 + c] -= (float)((double)ls + mu2 * (double)sm[c]);
-#pragma unroll
-    for (int c = 3; c < 6; c++) h[3 + c] -= (float)(mu2 * (double)sm[c]);
+    vis_atten<NM>(q, q.stage, id, lam, mu, h);
     // RK combine of the wave fields
     if (q.stage == 0) {
 #pragma unroll
@@ -150,7 +108,8 @@ static unsigned grid_for(long long n) {
 }
 
 int launch_vis_atten(const VisP &q, cudaStream_t st) {
-  const dim3 grid((q.ni + 127) / 128, q.nj, q.nk);
+  if (q.k0 >= q.nk) return 0;
+  const dim3 grid((q.ni + 127) / 128, q.nj, q.nk - q.k0);
   switch (q.nmax) {
     case 1: k_vis_atten<1><<<grid, 128, 0, st>>>(q); break;
     case 2: k_vis_atten<2><<<grid, 128, 0, st>>>(q); break;

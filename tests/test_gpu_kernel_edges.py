@@ -30,6 +30,12 @@ def _two_steps(p, shots=None, variant=None, setup=None):
     return [sim.wavefield(s) for s in range(sim.nshot)]
 
 
+def _close(a, b, tol):
+    for c in range(9):
+        scale = float(np.abs(b[c]).max())
+        assert float(np.abs(a[c] - b[c]).max()) <= tol * scale, f"component {c}"
+
+
 @pytest.mark.parametrize("medium", ["iso", "vti", "aniso", "ac"])
 @pytest.mark.parametrize("grid", GRIDS + [(101, 64, 48)])
 def test_default_chunk_changes_no_result(medium, grid):
@@ -96,3 +102,13 @@ def test_layer_averages_at_mixed_points(method, dims):
                 want = np.array([want[0], 1 / np.mean(1 / (v[:, 1] + 2 / 3 * v[:, 2])) - 2 / 3 * mu, mu])
         np.testing.assert_allclose(got[:, k, 1:-1, 1:-1], want[:, None, None] * np.ones((3, nj + 4, ni + 4)), rtol=5e-5)
     assert mixed >= 2
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("nmax", [1, 3, 4, 5])
+@pytest.mark.parametrize("free_top", [0, 1])
+def test_visco_fused_equals_separate_passes(nmax, grid, free_top):
+    p = small_problem("vis", *grid, nsteps=4, npml=3, free_top=free_top, nsrc=0)
+    p.visco["nmaxwell"] = nmax
+    (a,), (b,) = _two_steps(p), _two_steps(p, variant=0)
+    _close(a, b, 2e-5)
