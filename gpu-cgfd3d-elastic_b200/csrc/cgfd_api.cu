@@ -216,6 +216,7 @@ struct cgfd_problem {
 
   bool use_graph = true;
   bool use_tma = true;
+  bool tma64 = false;  // FP64 build, iso and VTI media: the TMA bulk kernel on doubles
   CUtensorMap map_halo[4], map_ctr[4], map_coef;  // acoustic media: the 4-field forms (make_ac_maps)
   bool ac_tma = false;  // acoustic FP32: the TMA-pipelined stage kernel (else the direct-load one)
   cudaGraphExec_t graph[8] = {};
@@ -329,6 +330,18 @@ struct cgfd_problem {
     return p;
   }
 
+  // tensor maps of one stage: the stage input, w_pre, w_end, coefficients
+  cgfd::TmaP stage_maps(int step, int s) const {
+    cgfd::TmaP tm;
+    const int pre = step & 1, end = (step + 1) & 1;
+    const int curs[4] = {pre, 2, 3, 2};
+    tm.cur = map_halo[curs[s]];
+    tm.pre = map_ctr[pre];
+    tm.end = map_ctr[end];
+    tm.coef = map_coef;
+    return tm;
+  }
+
   // Line receivers and slices: samples of w_pre at the start of the step, after the stations
   // (io_line_keep and io_slice_nc_put follow io_recv_keep, drv_rk_curv_col.cu:199-206).
   template <typename R>
@@ -352,22 +365,57 @@ struct cgfd_problem {
     return n;
   }
 
-  // One time step of the FP64 build: the same kernels instantiated in double (direct-load bulk
-  // kernel, surface slab, sources, stations, peak motion), launched in the same order.
+  // One time step of the FP64 build: the same kernels instantiated in double (bulk planes by TMA or,
+  // for 21-Cij media and cgfd_set_bulk_variant 0, by direct loads), launched in the same order and,
+  // with the TMA kernel, with the same work on the side stream as the FP32 step.
   int enqueue_step64(int step) {
     cudaStream_t st = stream;
     int n = 0;
-    if (rec.n > 0) {
-      cgfd::RecvPT<double> r;
-      r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-      r.pre = rptr<double>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
-      n += timed(6, [&] { return cgfd::launch_recv(r, st); });
-    }
-    n += enqueue_outputs<double>(step, st);
+    const bool fork = tma64 && tiles.n > 0 && !timing;
+    const bool early_peak = fork && free_top && !src_top;
+    auto sample = [&](cudaStream_t s2) {
+      int k = 0;
+      if (rec.n > 0) {
+        cgfd::RecvPT<double> r;
+        r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
+        r.pre = rptr<double>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+        k += timed(6, [&] { return cgfd::launch_recv(r, s2); });
+      }
+      return k + enqueue_outputs<double>(step, s2);
+    };
+    auto peak = [&](cudaStream_t s2) {
+      cgfd::PgPT<double> q;
+      q.ni = ni; q.nj = nj; q.nshot = nshot; q.sx = sx; q.sf = sf;
+      q.off_top = off0 + (long long)(nk - 1) * sz;
+      q.w_end = rptr<double>(wbuf[(step + 1) & 1]); q.w_pre = rptr<double>(wbuf[step & 1]);
+      q.pg = d_pg; q.dis = rptr<double>(d_dis); q.dt = dt;
+      return cgfd::launch_peak_motion(q, s2);
+    };
+    if (!fork) n += sample(st);
     for (int s = 0; s < 4; s++) {
       const cgfd::StagePT<double> p = stage_params_t<double>(step, s);
-      n += timed(s, [&] { return cgfd::launch_stage_bulk(med, p, nzc, st); });
-      n += timed(4, [&] { return cgfd::launch_timg_flux64(p, st) + cgfd::launch_stage_surface64(med, p, st); });
+      const bool beside = fork && (free_top || s == 0 || s == 3);
+      if (beside) {
+        CK(cudaEventRecord(ev_fork, st));
+        CK(cudaStreamWaitEvent(side, ev_fork, 0));
+      }
+      if (tma64) {
+        const cgfd::TmaP tm = stage_maps(step, s);
+        n += timed(s, [&] { return cgfd::launch_stage_bulk_tma64(med, p, tm, p.dir[2] ? tiles_dn : tiles, st); });
+      } else {
+        n += timed(s, [&] { return cgfd::launch_stage_bulk(med, p, nzc, st); });
+      }
+      const cudaStream_t top = beside ? side : st;
+      n += timed(4, [&] { return cgfd::launch_timg_flux64(p, top) + cgfd::launch_stage_surface64(med, p, top); });
+      if (beside) {
+        if (s == 0) n += sample(side);
+        if (s == 3) {
+          if (early_peak) n += peak(side);
+          n += cgfd::launch_advance(d_it, side);
+        }
+        CK(cudaEventRecord(ev_join, side));
+        CK(cudaStreamWaitEvent(st, ev_join, 0));
+      }
       if (src.nsrc > 0) {
         cgfd::SrcPT<double> q;
         memset(&q, 0, sizeof(q));
@@ -376,19 +424,12 @@ struct cgfd_problem {
         q.ca = p.ca; q.cb = p.cb;
         q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
         q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it;
+        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it; q.it_ahead = beside && s == 3;
         n += timed(5, [&] { return cgfd::launch_source(q, st); });
       }
     }
-    if (free_top) {
-      cgfd::PgPT<double> q;
-      q.ni = ni; q.nj = nj; q.nshot = nshot; q.sx = sx; q.sf = sf;
-      q.off_top = off0 + (long long)(nk - 1) * sz;
-      q.w_end = rptr<double>(wbuf[(step + 1) & 1]); q.w_pre = rptr<double>(wbuf[step & 1]);
-      q.pg = d_pg; q.dis = rptr<double>(d_dis); q.dt = dt;
-      n += cgfd::launch_peak_motion(q, st);
-    }
-    n += cgfd::launch_advance(d_it, st);
+    if (free_top && !early_peak) n += peak(st);
+    if (!fork) n += cgfd::launch_advance(d_it, st);
     return n;
   }
 
@@ -434,12 +475,7 @@ struct cgfd_problem {
         CK(cudaStreamWaitEvent(side, ev_fork, 0));
       }
       if (vis_tma) {
-        cgfd::TmaP tm;
-        const int curs[4] = {step & 1, 2, 3, 2};
-        tm.cur = map_halo[curs[s]];
-        tm.pre = map_ctr[step & 1];
-        tm.end = map_ctr[(step + 1) & 1];
-        tm.coef = map_coef;
+        const cgfd::TmaP tm = stage_maps(step, s);
         n += timed(s, [&] { return cgfd::launch_stage_bulk_vis(p, tm, v, p.dir[2] ? tiles_dn : tiles, st); });
       }
       p.rhs = d_rhs;
@@ -506,13 +542,7 @@ struct cgfd_problem {
         int t = -1;
         if constexpr (std::is_same<R, float>::value) {
           if (ac_tma) {
-            cgfd::TmaP tm;
-            const int pre = step & 1, end = (step + 1) & 1;
-            const int curs[4] = {pre, 2, 3, 2};
-            tm.cur = map_halo[curs[s]];
-            tm.pre = map_ctr[pre];
-            tm.end = map_ctr[end];
-            tm.coef = map_coef;
+            const cgfd::TmaP tm = stage_maps(step, s);
             t = cgfd::launch_stage_ac_tma(p, tm, nzc, st);
           }
         }
@@ -587,13 +617,7 @@ struct cgfd_problem {
         CK(cudaStreamWaitEvent(side, ev_fork, 0));
       }
       if (use_tma) {
-        cgfd::TmaP tm;
-        const int pre = step & 1, end = (step + 1) & 1;
-        const int curs[4] = {pre, 2, 3, 2};
-        tm.cur = map_halo[curs[s]];
-        tm.pre = map_ctr[pre];
-        tm.end = map_ctr[end];
-        tm.coef = map_coef;
+        const cgfd::TmaP tm = stage_maps(step, s);
         n += timed(s, [&] {
           return cgfd::launch_stage_bulk_tma(med, coef_type, wave16, shape, p, tm, p.dir[2] ? tiles_dn : tiles, st);
         });
@@ -1010,6 +1034,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
            : d->medium_type == CGFD_MEDIUM_ELASTIC_ISO ? cgfd::MED_ISO
            : (d->medium_type == CGFD_MEDIUM_ELASTIC_VTI ? cgfd::MED_VTI : cgfd::MED_ANISO);
   p->ncoef = p->med == cgfd::MED_AC ? 11 : (p->med == cgfd::MED_ISO ? 12 : (p->med == cgfd::MED_VTI ? 15 : 31));
+  p->tma64 = p->fp64 && cgfd::tma64_supported(p->med);
   if (p->med == cgfd::MED_AC) {  // acoustic media run their own stage kernel (TMA-pipelined in FP32)
     p->use_tma = false;
     p->ac_tma = !p->fp64;
@@ -1079,7 +1104,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
   if (p->coef_type != cgfd::COEF_F32) to_16bit_coefficients(p);
 
   // TMA tensor maps of the four wavefield levels and of the coefficients
-  if (p->use_tma || p->vis_tma) make_maps(p);
+  if (p->use_tma || p->vis_tma || p->tma64) make_maps(p);
   if (p->ac_tma) make_ac_maps(p);
   // free surface of elastic media: velocity-gradient conversion and traction-image fluxes
   if (p->free_top && p->med != cgfd::MED_AC) {
@@ -1264,7 +1289,19 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
 // shape (box heights follow the tile), and the bulk kernels' shared-memory attributes.
 void make_maps(cgfd_problem *p) {
   const int nshot = p->nshot;
-  {
+  if (p->tma64) {  // every level and the coefficients in double
+    const int ty = cgfd::tma64_tile_y(p->med);
+    const auto f64 = CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
+    for (int l = 0; l < 4; l++) {
+      make_map(&p->map_halo[l], p->rvoid(p->wbuf[l], p->off0), p->ni, p->nj, p->nk, 9 * nshot, p->sx, p->sz, p->sf,
+               cgfd::TX + 8, ty + 4, 9, f64, 8);
+      make_map(&p->map_ctr[l], p->wbuf[l], p->sx, p->nj + 6, p->nk + 6, 9 * nshot, p->sx, p->sz, p->sf, cgfd::TX, ty, 9,
+               f64, 8);
+    }
+    make_map(&p->map_coef, p->coef, p->sx, p->nj + 6, p->nk + 6, p->ncoef, p->sx, p->sz, p->sf, cgfd::TX, ty, p->ncoef,
+             f64, 8);
+    CK(cgfd::tma64_prepare(p->med));
+  } else {
     const int ty = cgfd::tma_tile_y(p->med, p->shape);
     // The stage-input (halo) maps cover the physical cells only, from (0, 0, 0): the halo columns,
     // rows and planes beyond the grid, which hold zeros in memory, come as the boxes' zero fill
@@ -1389,14 +1426,14 @@ int default_chunk(const cgfd_problem *p) {
 // (tiles), downwards for forward ones (tiles_dn).
 void make_tiles(cgfd_problem *p) {
   if (p->med == cgfd::MED_AC) return;  // no TMA kernel for acoustic media
-  const int ty = cgfd::tma_tile_y(p->med, p->shape);
+  const int ty = p->tma64 ? cgfd::tma64_tile_y(p->med) : cgfd::tma_tile_y(p->med, p->shape);
   const int nbx = (p->ni + cgfd::TX - 1) / cgfd::TX, nby = (p->nj + ty - 1) / ty;
   if (nbx > cgfd::kTileBxMask + 1) throw cgfd::Error(CGFD_ERR_INVALID, "grid too wide for the bulk tile list");
   const auto zr = z_ranges(p, p->nzc);
   int nsm = 148;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
   const int group = std::max(1, std::min(p->shot_group, p->nshot));
-  const long long resident = (long long)nsm * cgfd::tma_blocks_per_sm(p->med, p->shape);
+  const long long resident = (long long)nsm * (p->tma64 ? cgfd::tma64_resident(p->med) : cgfd::tma_blocks_per_sm(p->med, p->shape));
   const int strip = (int)std::max<long long>(1, (resident + (long long)nbx * group - 1) / ((long long)nbx * group));
   for (int dn = 0; dn < 2; dn++) {
     std::vector<int4> list;
@@ -2122,7 +2159,7 @@ int cgfd_set_bulk_variant(cgfd_problem *p, int tma) {
     return CGFD_ERR_UNSUPPORTED;
   }
   p->use_tma = tma != 0;
-  p->vis_tma = false;  // visco-elastic media come here with 0 only
+  p->vis_tma = p->tma64 = false;  // visco-elastic media and the FP64 build come here with 0 only
   for (int s = 0; s < 8; s++)
     if (p->graph_ok[s]) { cudaGraphExecDestroy(p->graph[s]); p->graph_ok[s] = false; }
   return CGFD_OK;

@@ -29,9 +29,10 @@ namespace cgfd {
 // Wave policies: stage input / next-stage output storage.
 //   WP 0: FP32 in, FP32 out (plain)      WP 1: FP32 in, FP16 out (stage 0 of FP16 mode)
 //   WP 2: FP16 in, FP16 out (stages 1-3 of FP16 mode; stage 3 has no stage output)
-template <int WP> struct WavePolicy {
-  using TW = typename std::conditional<WP == 2, __half, float>::type;
-  using TT = typename std::conditional<WP >= 1, __half, float>::type;
+// R: the real type of everything else (double in the FP64 build, WP 0).
+template <int WP, typename R = float> struct WavePolicy {
+  using TW = typename std::conditional<WP == 2, __half, R>::type;
+  using TT = typename std::conditional<WP >= 1, __half, R>::type;
 };
 
 // Tile shapes (columns x rows of one thread block, resident blocks per SM), two per medium; the
@@ -50,7 +51,8 @@ template <> struct TileShape<MED_ANISO, 1> { static constexpr int TYT = 8, MINB 
 
 template <int MED, int TYT, typename TC, typename TW, int MINB>
 struct BulkSmem {
-  static constexpr int XO = 16 / (int)sizeof(TW);  // x halo of the box: 16 bytes, TMA-aligned
+  // x halo of the box: 3 points at least, a multiple of 16 bytes (TMA alignment)
+  static constexpr int XO = sizeof(TW) == 8 ? 4 : 16 / (int)sizeof(TW);
   static constexpr int WX = TX + 2 * XO;  // x box [-XO, 32+XO) around the tile
   static constexpr int WY = TYT + 4;      // y box [-1, TYT+3) (forward) or [-3, TYT+1) (backward)
   static constexpr int NC = MedInfo<MED>::NCOEF;
@@ -58,10 +60,10 @@ struct BulkSmem {
   static constexpr int WAVE_ELEMS = 9 * WY * WX;
   static constexpr int WAVE_SLOT = ((WAVE_ELEMS * (int)sizeof(TW) + 127) / 128) * 128;  // bytes
   static constexpr int COEF_BYTES = NC * CELLS * (int)sizeof(TC);  // multiple of 128 for every medium
-  static constexpr int FLD_BYTES = 9 * CELLS * 4;
+  static constexpr int FLD_BYTES = 9 * CELLS * (int)sizeof(real_of<TC>);
   // w_pre staged by TMA at one block per SM; with two blocks per SM it is read directly
   // (measured faster on 480x480x240: the smaller ring leaves the SM more L1)
-  static constexpr bool PT = MINB == 1;
+  static constexpr bool PT = MINB == 1 && sizeof(real_of<TC>) == 4;
   static constexpr int OFF_END = COEF_BYTES + (PT ? FLD_BYTES : 0);  // within a cpe slot
   static constexpr int CPE_SLOT = OFF_END + FLD_BYTES;
   static constexpr int NW = 3;  // wave ring slots: this plane, the one ahead, one in flight
@@ -81,17 +83,18 @@ struct BulkSmem {
 template <typename TC, int STRIDE>
 struct CoefTile {
   const TC *c;  // field 0 of this cell
-  const StageP &p;
-  __device__ __forceinline__ float operator()(int f) const { return coef_decode<TC>(c[f * STRIDE], p, f); }
+  const StagePT<real_of<TC>> &p;
+  __device__ __forceinline__ real_of<TC> operator()(int f) const { return coef_decode<TC>(c[f * STRIDE], p, f); }
 };
 
 // One tile (a block) of the stage; PML false: the tile meets no CFS-PML face and the face code
 // is compiled out.
 // VIS: the visco-elastic form with that many mechanisms (0: elastic; vp is then unused).
 template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP, bool PML, int VIS = 0>
-__device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const int4 tl, const VisP *vp = nullptr) {
-  using TW = typename WavePolicy<WP>::TW;
-  using TT = typename WavePolicy<WP>::TT;
+__device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const TmaP &tm, const int4 tl, const VisP *vp = nullptr) {
+  using R = real_of<TC>;
+  using TW = typename WavePolicy<WP, R>::TW;
+  using TT = typename WavePolicy<WP, R>::TT;
   using S = BulkSmem<MED, TYT, TC, TW, MINB>;
   constexpr int LX = op_left(DX), LY = op_left(DY);
   constexpr int SD = DZ ? -1 : 1;  // march direction
@@ -113,7 +116,7 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
   const long long woff = (long long)shot * 9 * sf;
   const TW *__restrict__ cur = reinterpret_cast<const TW *>(p.cur) + woff;
   TT *__restrict__ tmp_out = reinterpret_cast<TT *>(p.tmp_out) + woff;
-  float *__restrict__ endw = p.end + woff;
+  R *__restrict__ endw = p.end + woff;
   const int stage = p.stage;
   const bool need_pre = stage == 1 || stage == 2;
   const bool need_end = stage >= 1;
@@ -159,7 +162,7 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
   // are cut at the z faces, so a column's faces are the same at every plane of the tile
   unsigned fmask = 0, tmask = 0;
   for (int fi = 0; PML && fi < p.nface; fi++) {
-    const FaceP &f = p.face[fi];
+    const FacePT<R> &f = p.face[fi];
     const bool xo = f.lo[0] <= bx * TX + TX - 1 && f.hi[0] >= bx * TX;
     const bool yo = f.lo[1] <= by * TYT + TYT - 1 && f.hi[1] >= by * TYT;
     const bool zo = f.lo[2] <= ke - 1 && f.hi[2] >= kb;
@@ -168,11 +171,11 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
   }
 
   // register queue of the planes behind, in march order: q[f][n] = plane k + (n - 3) * SD
-  float q[9][3];
+  R q[9][3];
 #pragma unroll
   for (int f = 0; f < 9; f++)
 #pragma unroll
-    for (int m = 0; m < 3; m++) q[f][m] = 0.f;
+    for (int m = 0; m < 3; m++) q[f][m] = R(0);
   if (act) {
 #pragma unroll
     for (int m = 0; m < 3; m++) {
@@ -201,43 +204,43 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
 
     if (act) {
       const CoefTile<TC, S::CELLS> Cc{reinterpret_cast<const TC *>(cpe + cs * S::CPE_SLOT) + cell, p};
-      float mt[3][3];
+      R mt[3][3];
 #pragma unroll
       for (int a = 0; a < 3; a++)
 #pragma unroll
         for (int b = 0; b < 3; b++) mt[a][b] = Cc(3 * a + b);
-      const float slw = Cc(CF_SLW);
-      Medium<MED> md;
+      const R slw = Cc(CF_SLW);
+      Medium<MED, R> md;
       md.load(Cc);
       // the 9 derivatives of the stage input along one axis at this cell
-      auto deriv_x = [&](float d[9]) {
+      auto deriv_x = [&](R d[9]) {
 #pragma unroll
         for (int f = 0; f < 9; f++) {
           const TW *r = W + f * S::WY * S::WX + (ty + LY) * S::WX + tx + S::XO - LX;
           d[f] = drp5<DX>(to_f(r[0]), to_f(r[1]), to_f(r[2]), to_f(r[3]), to_f(r[4]));
-          if constexpr (WP == 2) d[f] *= s_wsc[f];  // the operator is linear: scale once
+          if constexpr (WP == 2) d[f] *= R(s_wsc[f]);  // the operator is linear: scale once
         }
       };
-      auto deriv_y = [&](float d[9]) {
+      auto deriv_y = [&](R d[9]) {
 #pragma unroll
         for (int f = 0; f < 9; f++) {
           const TW *r = W + f * S::WY * S::WX + ty * S::WX + tx + S::XO;
           d[f] = drp5<DY>(to_f(r[0]), to_f(r[S::WX]), to_f(r[2 * S::WX]), to_f(r[3 * S::WX]), to_f(r[4 * S::WX]));
-          if constexpr (WP == 2) d[f] *= s_wsc[f];
+          if constexpr (WP == 2) d[f] *= R(s_wsc[f]);
         }
       };
-      auto deriv_z = [&](float d[9]) {  // queue, this plane and the one ahead, in increasing k
+      auto deriv_z = [&](R d[9]) {  // queue, this plane and the one ahead, in increasing k
 #pragma unroll
         for (int f = 0; f < 9; f++) {
-          const float c0 = to_f(W[f * S::WY * S::WX + wc]), c1 = to_f(Wn[f * S::WY * S::WX + wc]);
+          const R c0 = to_f(W[f * S::WY * S::WX + wc]), c1 = to_f(Wn[f * S::WY * S::WX + wc]);
           d[f] = SD > 0 ? drp5<DZ>(q[f][0], q[f][1], q[f][2], c0, c1) : drp5<DZ>(c1, c0, q[f][2], q[f][1], q[f][0]);
-          if constexpr (WP == 2) d[f] *= s_wsc[f];
+          if constexpr (WP == 2) d[f] *= R(s_wsc[f]);
         }
       };
-      CellAcc acc;
+      CellAcc<R> acc;
       acc.zero();
       {
-        float d[9];
+        R d[9];
         deriv_x(d);
         acc.add_axis(mt[0], d, d + 3);
         deriv_y(d);
@@ -245,7 +248,7 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
         deriv_z(d);
         acc.add_axis(mt[2], d, d + 3);
       }
-      float h[9];
+      R h[9];
       h[0] = slw * acc.mom[0];
       h[1] = slw * acc.mom[1];
       h[2] = slw * acc.mom[2];
@@ -258,8 +261,8 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
         for (unsigned left = fmask; left; left &= left - 1) {
           const int fi = __ffs(left) - 1;
           if (!(tmask >> fi & 1)) continue;
-          const FaceP &fc = p.face[fi];
-          float d[9];
+          const FacePT<R> &fc = p.face[fi];
+          R d[9];
           if (fc.axis == 0) {
             deriv_x(d);
             pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[0], d, d + 3, nullptr, nullptr, h, shot);
@@ -275,34 +278,34 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
       const long long id = didx(p, i, j, k);
       if constexpr (VIS > 0) vis_atten<VIS>(*vp, stage, id, md.lam, md.mu, h);
       // RK combine (wav_update / wav_update_end)
-      const float *PR = reinterpret_cast<const float *>(cpe + cs * S::CPE_SLOT + S::COEF_BYTES) + cell;
-      const float *EN = reinterpret_cast<const float *>(cpe + cs * S::CPE_SLOT + S::OFF_END) + cell;
-      const float *prg = p.pre + woff + id;  // w_pre in HBM when it is not staged
-      const float ca = p.ca, cb = p.cb;
+      const R *PR = reinterpret_cast<const R *>(cpe + cs * S::CPE_SLOT + S::COEF_BYTES) + cell;
+      const R *EN = reinterpret_cast<const R *>(cpe + cs * S::CPE_SLOT + S::OFF_END) + cell;
+      const R *prg = p.pre + woff + id;  // w_pre in HBM when it is not staged
+      const R ca = p.ca, cb = p.cb;
       if (stage == 0) {
 #pragma unroll
         for (int f = 0; f < 9; f++) {
-          const float c0 = to_f(W[f * S::WY * S::WX + wc]);  // stage input = w_pre at stage 0
-          const float t = c0 + ca * h[f];
-          tmp_out[f * sf + id] = from_f<TT>(WP != 0 ? t * s_wsc[9 + f] : t);
+          const R c0 = to_f(W[f * S::WY * S::WX + wc]);  // stage input = w_pre at stage 0
+          const R t = c0 + ca * h[f];
+          tmp_out[f * sf + id] = from_f<TT>(WP != 0 ? t * R(s_wsc[9 + f]) : t);
           endw[f * sf + id] = c0 + cb * h[f];
         }
       } else if (stage < 3) {
 #pragma unroll
         for (int f = 0; f < 9; f++) {
-          const float t = (S::PT ? PR[f * S::CELLS] : __ldg(prg + f * sf)) + ca * h[f];
-          tmp_out[f * sf + id] = from_f<TT>(WP != 0 ? t * s_wsc[9 + f] : t);
+          const R t = (S::PT ? PR[f * S::CELLS] : __ldg(prg + f * sf)) + ca * h[f];
+          tmp_out[f * sf + id] = from_f<TT>(WP != 0 ? t * R(s_wsc[9 + f]) : t);
           endw[f * sf + id] = EN[f * S::CELLS] + cb * h[f];
         }
       } else {
 #pragma unroll
         for (int f = 0; f < 9; f++) {
-          const float e = EN[f * S::CELLS] + cb * h[f];
+          const R e = EN[f * S::CELLS] + cb * h[f];
           endw[f * sf + id] = e;
           bad |= nonfinite(e);
           if constexpr (WP == 2) {
-            if (f < 3) vmax = fmaxf(vmax, fabsf(e));
-            else smax = fmaxf(smax, fabsf(e));
+            if (f < 3) vmax = fmaxf(vmax, fabsf((float)e));
+            else smax = fmaxf(smax, fabsf((float)e));
           }
         }
       }
@@ -339,8 +342,8 @@ __device__ __forceinline__ void bulk_tile(const StageP &p, const TmaP &tm, const
 // others its compiled-out form. Both kinds in one launch keep a tile's x-y neighbours, PML or
 // not, resident beside it, so that the halo lines they share are read from DRAM once.
 template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP>
-__global__ void __launch_bounds__(TX *TYT, BulkSmem<MED, TYT, TC, typename WavePolicy<WP>::TW, MINB>::BOUND)
-    k_stage_bulk_tma(const __grid_constant__ StageP p, const __grid_constant__ TmaP tm,
+__global__ void __launch_bounds__(TX *TYT, BulkSmem<MED, TYT, TC, typename WavePolicy<WP, real_of<TC>>::TW, MINB>::BOUND)
+    k_stage_bulk_tma(const __grid_constant__ StagePT<real_of<TC>> p, const __grid_constant__ TmaP tm,
                      const int4 *__restrict__ tiles) {
   const int4 tl = __ldg(tiles + blockIdx.x);
   if (tl.x & kTilePml) bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, true>(p, tm, tl);

@@ -168,6 +168,12 @@ struct BulkTiles {
 };
 int launch_stage_bulk_tma(int med, int coef_type, int wave16, int shape, const StageP &p, const TmaP &tm,
                           const BulkTiles &t, cudaStream_t st);
+// The FP64 build's TMA bulk kernel (iso and VTI media)
+bool tma64_supported(int med);
+int tma64_tile_y(int med);
+int tma64_resident(int med);
+cudaError_t tma64_prepare(int med);
+int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st);
 // The visco-elastic form of the bulk kernel: the iso stage with the attenuation of the point and the
 // RK combine of the memory variables (v) between the right-hand side and the combine (32x4 tiles), for
 // up to vis_bulk_max_mechanisms() mechanisms (media with more run the direct-load kernel and the

@@ -8,7 +8,7 @@ equal to double rounding, so their read-back floats differ by one unit in the la
 import numpy as np
 import pytest
 
-from cgfd_b200 import Simulation, media_layer_gpu, CGFD_MEDIA_ARI, CGFD_MEDIA_HAR
+from cgfd_b200 import Simulation, media_layer_gpu, CGFD_MEDIA_ARI, CGFD_MEDIA_HAR, CGFD_PREC_FP64
 from cgfd_b200.formats import LayerModel
 from helpers import small_problem, random_wavefield
 
@@ -112,3 +112,13 @@ def test_visco_fused_equals_separate_passes(nmax, grid, free_top):
     p.visco["nmaxwell"] = nmax
     (a,), (b,) = _two_steps(p), _two_steps(p, variant=0)
     _close(a, b, 2e-5)
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("medium", ["iso", "vti"])
+@pytest.mark.parametrize("free_top", [0, 1])
+def test_fp64_tma_equals_direct(medium, grid, free_top):
+    p = small_problem(medium, *grid, nsteps=4, npml=3, free_top=free_top, nsrc=0)
+    p.precision = CGFD_PREC_FP64
+    (a,), (b,) = _two_steps(p), _two_steps(p, variant=0)
+    _close(a, b, 1.2e-7)
