@@ -305,9 +305,9 @@ struct AcSmem {
   static_assert(MINB * (BYTES + 1024) <= 228 * 1024, "MINB blocks must fit one SM's shared memory");
 };
 
-template <int DX, int DY, int DZ>
-__global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
-    k_stage_ac_tma(const __grid_constant__ StageP p, const __grid_constant__ TmaP tm, int nzc, int nchunk) {
+// One tile (a block); PML false: no CFS-PML face meets it and the face code is compiled out.
+template <int DX, int DY, int DZ, bool PML>
+__device__ __forceinline__ void ac_tile(const StageP &p, const TmaP &tm, const int4 tl) {
   using S = AcSmem;
   constexpr int TYT = S::TYT;
   constexpr int LX = op_left(DX), LY = op_left(DY);
@@ -318,9 +318,8 @@ __global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + S::OFF_BAR);  // NW wave, then 2 cpe
 
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int bx = blockIdx.x, by = blockIdx.y;
-  const int shot = blockIdx.z / nchunk, kb = (blockIdx.z % nchunk) * nzc;
-  const int ke = min(kb + nzc, p.nk);
+  const int bx = tl.x & kTileBxMask, by = tl.y, shot = tl.x >> 16;
+  const int kb = tl.z, ke = tl.w;
   if (kb >= ke) return;
   const int n = ke - kb;
   const int i = bx * TX + tx, j = by * TYT + ty;
@@ -368,14 +367,16 @@ __global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
     issue_cpe(0);
   }
 
-  // PML faces that intersect this block (uniform)
-  unsigned fmask = 0;
-  for (int fi = 0; fi < p.nface; fi++) {
+  // PML faces that intersect this block (uniform), and those this thread's column lies in (z chunks
+  // are cut at the z faces)
+  unsigned fmask = 0, tmask = 0;
+  for (int fi = 0; PML && fi < p.nface; fi++) {
     const FaceP &f = p.face[fi];
     const bool xo = f.lo[0] <= bx * TX + TX - 1 && f.hi[0] >= bx * TX;
     const bool yo = f.lo[1] <= by * TYT + TYT - 1 && f.hi[1] >= by * TYT;
     const bool zo = f.lo[2] <= ke - 1 && f.hi[2] >= kb;
     if (xo && yo && zo) fmask |= 1u << fi;
+    if (act && in_face(f, i, j, k0)) tmask |= 1u << fi;
   }
 
   // register queue of the planes behind, in march order: q[f][n] = plane k + (n - 3) * SD
@@ -454,11 +455,12 @@ __global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
                         : -kappa * (mt[0][0] * dv[0][0] + mt[1][0] * dv[1][0] + mt[2][0] * dvz[0] +
                                     mt[0][1] * dv[0][1] + mt[1][1] * dv[1][1] + mt[2][1] * dvz[1] +
                                     mt[0][2] * dv[0][2] + mt[1][2] * dv[1][2] + mt[2][2] * dvz[2]);
-      if (fmask) {
+      if (PML && tmask) {
         float hc[kAcF] = {0.f, 0.f, 0.f, 0.f};
-        for (int fi = 0; fi < p.nface; fi++) {
+        for (unsigned left = fmask; left; left &= left - 1) {
+          const int fi = __ffs(left) - 1;
+          if (!(tmask >> fi & 1)) continue;
           const FaceP &fc = p.face[fi];
-          if (!(fmask >> fi & 1) || !in_face(fc, i, j, k)) continue;
           // (an index into the register arrays by fc.axis would put them in local memory for every
           // cell, PML or not)
           if (fc.axis == 0) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[0], dv[0], dp[0], hc);
@@ -508,22 +510,36 @@ __global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
   if (bad) atomicOr(p.err, kErrWaveNonfinite);
 }
 
-int launch_stage_ac_tma(const StageP &p, const TmaP &tm, int nzc, cudaStream_t st) {
-  nzc = std::max(1, std::min(nzc, p.nk));
-  const int nchunk = (p.nk + nzc - 1) / nzc;
-  if ((long long)nchunk * p.nshot > 65535) return -1;  // the caller runs the direct-load kernel
+// One block per tile-list entry, in list order (strips of tile rows in z layers along the march, as
+// the elastic bulk kernel: a tile's neighbours run beside it and share its halo lines in L2).
+template <int DX, int DY, int DZ>
+__global__ void __launch_bounds__(TX *AcSmem::TYT, AcSmem::MINB)
+    k_stage_ac_tma(const __grid_constant__ StageP p, const __grid_constant__ TmaP tm, const int4 *__restrict__ tiles) {
+  const int4 tl = __ldg(tiles + blockIdx.x);
+  if (tl.x & kTilePml) ac_tile<DX, DY, DZ, true>(p, tm, tl);
+  else ac_tile<DX, DY, DZ, false>(p, tm, tl);
+}
+
+int ac_tma_resident() { return AcSmem::MINB; }
+
+cudaError_t ac_tma_prepare() {
+  cudaError_t e = cudaSuccess;
+#define ATTR(c)                                                                                  \
+  if (e == cudaSuccess)                                                                          \
+    e = cudaFuncSetAttribute(k_stage_ac_tma<(c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1>,              \
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, AcSmem::BYTES);
+  ATTR(0) ATTR(1) ATTR(2) ATTR(3) ATTR(4) ATTR(5) ATTR(6) ATTR(7)
+#undef ATTR
+  return e;
+}
+
+int launch_stage_ac_tma(const StageP &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st) {
+  if (t.n <= 0) return 0;
   const dim3 block(TX, AcSmem::TYT);
-  const dim3 grid((p.ni + TX - 1) / TX, (p.nj + AcSmem::TYT - 1) / AcSmem::TYT, nchunk * p.nshot);
-  static bool attr_done[8] = {};  // the opt-in above 48 KB of dynamic shared memory, once per instantiation
   switch (p.dir[0] | (p.dir[1] << 1) | (p.dir[2] << 2)) {
 #define CASE(c)                                                                                           \
   case c:                                                                                                 \
-    if (!attr_done[c]) {                                                                                  \
-      cudaFuncSetAttribute(k_stage_ac_tma<(c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1>,                         \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, AcSmem::BYTES);                   \
-      attr_done[c] = true;                                                                                \
-    }                                                                                                     \
-    k_stage_ac_tma<(c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1><<<grid, block, AcSmem::BYTES, st>>>(p, tm, nzc, nchunk); \
+    k_stage_ac_tma<(c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1><<<t.n, block, AcSmem::BYTES, st>>>(p, tm, t.list); \
     break;
     CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7)
 #undef CASE

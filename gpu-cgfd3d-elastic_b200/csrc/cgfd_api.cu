@@ -218,6 +218,7 @@ struct cgfd_problem {
   bool use_tma = true;
   bool tma64 = false;  // FP64 build, iso and VTI media: the TMA bulk kernel on doubles
   CUtensorMap map_halo[4], map_ctr[4], map_coef;  // acoustic media: the 4-field forms (make_ac_maps)
+  bool ac_tiled = false;  // acoustic FP32: maps and tile lists of the TMA stage kernel exist
   bool ac_tma = false;  // acoustic FP32: the TMA-pipelined stage kernel (else the direct-load one)
   cudaGraphExec_t graph[8] = {};
   bool graph_ok[8] = {};
@@ -328,6 +329,24 @@ struct cgfd_problem {
       o.cur = stage == 0 ? o.pre : o.tmp;
     }
     return p;
+  }
+
+  // whether the bulk (acoustic: whole) stage runs from tile lists; tile height, and blocks per SM of
+  // the kernel that does (strip_blocks: those the strips of the tile order are sized for)
+  bool tiled() const { return med != cgfd::MED_AC || ac_tiled; }
+  int tile_y() const {
+    return med == cgfd::MED_AC ? cgfd::TY : tma64 ? cgfd::tma64_tile_y(med) : cgfd::tma_tile_y(med, shape);
+  }
+  int strip_blocks() const {
+    return med == cgfd::MED_AC ? cgfd::ac_tma_resident()
+                               : tma64 ? cgfd::tma64_resident(med) : cgfd::tma_blocks_per_sm(med, shape);
+  }
+  int resident_blocks() const {
+    if (med == cgfd::MED_AC) return fp64 ? 1 : cgfd::ac_tma_resident();
+    if (tma64) return cgfd::tma64_resident(med);
+    if (fp64) return 1;
+    if (vis) return vis_tma ? cgfd::tma_blocks_per_sm(med, shape) : 2;
+    return cgfd::tma_resident(med, coef_type, wave16, shape);
   }
 
   // tensor maps of one stage: the stage input, w_pre, w_end, coefficients
@@ -538,15 +557,10 @@ struct cgfd_problem {
     for (int s = 0; s < 4; s++) {
       const cgfd::StagePT<R> p = stage_params_t<R>(step, s);
       n += timed(s, [&] {
-        int k = cgfd::launch_ac_image(p, st);
-        int t = -1;
-        if constexpr (std::is_same<R, float>::value) {
-          if (ac_tma) {
-            const cgfd::TmaP tm = stage_maps(step, s);
-            t = cgfd::launch_stage_ac_tma(p, tm, nzc, st);
-          }
-        }
-        return k + (t >= 0 ? t : cgfd::launch_stage_ac(p, nzc, st));
+        const int k = cgfd::launch_ac_image(p, st);
+        if constexpr (std::is_same<R, float>::value)
+          if (ac_tma) return k + cgfd::launch_stage_ac_tma(p, stage_maps(step, s), p.dir[2] ? tiles_dn : tiles, st);
+        return k + cgfd::launch_stage_ac(p, nzc, st);
       });
       if (src.nsrc > 0) {
         cgfd::SrcPT<R> q;
@@ -1037,7 +1051,9 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
   p->tma64 = p->fp64 && cgfd::tma64_supported(p->med);
   if (p->med == cgfd::MED_AC) {  // acoustic media run their own stage kernel (TMA-pipelined in FP32)
     p->use_tma = false;
-    p->ac_tma = !p->fp64;
+    // (a grid of more tile columns than a tile-list entry numbers runs the direct-load kernel)
+    p->ac_tma = !p->fp64 && (p->ni + cgfd::TX - 1) / cgfd::TX <= cgfd::kTileBxMask + 1;
+    p->ac_tiled = p->ac_tma;
   }
   p->nt_total = d->nt_total;
   p->dt = d->dt;
@@ -1348,6 +1364,7 @@ void make_ac_maps(cgfd_problem *p) {
   }
   make_map(&p->map_coef, p->coef, p->sx, p->nj + 6, p->nk + 6, p->ncoef, p->sx, p->sz, p->sf, cgfd::TX, cgfd::TY,
            p->ncoef);
+  CK(cgfd::ac_tma_prepare());
 }
 
 // z ranges of the tile list: [0, nbulk) cut at the z-face boundaries of the CFS-PML, each part split
@@ -1381,11 +1398,9 @@ int default_chunk(const cgfd_problem *p) {
   if (p->nbulk < 1) return 1;
   int nsm = 148;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
-  const bool tiled = p->use_tma;
-  const int ty = tiled ? cgfd::tma_tile_y(p->med, p->shape) : cgfd::TY;
-  const int per_sm = tiled ? cgfd::tma_resident(p->med, p->coef_type, p->wave16, p->shape)
-                           : p->fp64 ? 1 : p->med == cgfd::MED_AC ? 3 : 2;
-  const long long resident = (long long)nsm * per_sm;
+  const bool tiled = p->use_tma || p->vis_tma || p->tma64 || p->ac_tma;
+  const int ty = tiled ? p->tile_y() : cgfd::TY;
+  const long long resident = (long long)nsm * p->resident_blocks();
   const long long columns = (long long)((p->ni + cgfd::TX - 1) / cgfd::TX) * ((p->nj + ty - 1) / ty) * p->nshot;
   auto even = [&](int c) {  // the chunk length of nbulk planes in equal chunks of at most c
     const int n = (p->nbulk + c - 1) / c;
@@ -1425,15 +1440,15 @@ int default_chunk(const cgfd_problem *p) {
 // layers run in the march direction of the stage's z operator: upwards for backward operators
 // (tiles), downwards for forward ones (tiles_dn).
 void make_tiles(cgfd_problem *p) {
-  if (p->med == cgfd::MED_AC) return;  // no TMA kernel for acoustic media
-  const int ty = p->tma64 ? cgfd::tma64_tile_y(p->med) : cgfd::tma_tile_y(p->med, p->shape);
+  if (!p->tiled()) return;
+  const int ty = p->tile_y();
   const int nbx = (p->ni + cgfd::TX - 1) / cgfd::TX, nby = (p->nj + ty - 1) / ty;
   if (nbx > cgfd::kTileBxMask + 1) throw cgfd::Error(CGFD_ERR_INVALID, "grid too wide for the bulk tile list");
   const auto zr = z_ranges(p, p->nzc);
   int nsm = 148;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
   const int group = std::max(1, std::min(p->shot_group, p->nshot));
-  const long long resident = (long long)nsm * (p->tma64 ? cgfd::tma64_resident(p->med) : cgfd::tma_blocks_per_sm(p->med, p->shape));
+  const long long resident = (long long)nsm * p->strip_blocks();
   const int strip = (int)std::max<long long>(1, (resident + (long long)nbx * group - 1) / ((long long)nbx * group));
   for (int dn = 0; dn < 2; dn++) {
     std::vector<int4> list;
@@ -2149,7 +2164,7 @@ int cgfd_set_bulk_variant(cgfd_problem *p, int tma) {
     return CGFD_ERR_UNSUPPORTED;
   }
   if (p->med == cgfd::MED_AC) {  // acoustic: the TMA-pipelined (1) or direct-load (0) stage kernel
-    p->ac_tma = tma != 0;
+    p->ac_tma = tma != 0 && p->ac_tiled;
     for (int s = 0; s < 8; s++)
       if (p->graph_ok[s]) { cudaGraphExecDestroy(p->graph[s]); p->graph_ok[s] = false; }
     return CGFD_OK;

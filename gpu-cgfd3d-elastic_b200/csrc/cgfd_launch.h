@@ -141,9 +141,6 @@ template <typename R>
 int launch_ac_image(const StagePT<R> &p, cudaStream_t st);
 template <typename R>
 int launch_stage_ac(const StagePT<R> &p, int nzc, cudaStream_t st);
-// the TMA-pipelined acoustic stage (FP32; tm: the acoustic maps of the stage input, w_pre,
-// w_end and the coefficients); -1 when the grid does not fit one launch (run launch_stage_ac)
-int launch_stage_ac_tma(const StageP &p, const TmaP &tm, int nzc, cudaStream_t st);
 // FP64 build: the surface slab with double storage and arithmetic
 int launch_stage_surface64(int med, const StagePT<double> &p, cudaStream_t st);
 // traction-image fluxes of the stage input for the surface slab (before it, same stream)
@@ -166,6 +163,10 @@ struct BulkTiles {
   const int4 *list = nullptr;
   int n = 0, npml = 0;  // entries, of which PML tiles
 };
+// the TMA-pipelined acoustic stage (FP32; tm: the acoustic maps; 32 x TY tiles of every plane)
+int ac_tma_resident();
+cudaError_t ac_tma_prepare();
+int launch_stage_ac_tma(const StageP &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st);
 int launch_stage_bulk_tma(int med, int coef_type, int wave16, int shape, const StageP &p, const TmaP &tm,
                           const BulkTiles &t, cudaStream_t st);
 // The FP64 build's TMA bulk kernel (iso and VTI media)

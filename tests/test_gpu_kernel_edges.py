@@ -122,3 +122,13 @@ def test_fp64_tma_equals_direct(medium, grid, free_top):
     p.precision = CGFD_PREC_FP64
     (a,), (b,) = _two_steps(p), _two_steps(p, variant=0)
     _close(a, b, 1.2e-7)
+
+
+@pytest.mark.parametrize("grid", GRIDS)
+@pytest.mark.parametrize("free_top", [0, 1])
+@pytest.mark.parametrize("nshot", [1, 3])
+def test_acoustic_tiles_equal_direct(grid, free_top, nshot):
+    p = small_problem("ac", *grid, nsteps=4, npml=3, free_top=free_top, nsrc=1)
+    shots = [p.src] * nshot if nshot > 1 else None
+    for a, b in zip(_two_steps(p, shots), _two_steps(p, shots, variant=0)):
+        _close(a, b, 2e-5)  # components 4-8 stay 0 in both
