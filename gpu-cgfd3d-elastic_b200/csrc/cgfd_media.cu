@@ -21,10 +21,12 @@
 
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cgfd_b200.h"
 #include "cgfd_setup.h"
+#include "cgfd_stager.h"
 
 namespace cgfd {
 namespace {
@@ -44,27 +46,44 @@ struct P3 {
   float x, y, z;
 };
 
-// BilinearInterpolation (media_utility.cpp:325-360) on the uniform interface mesh; FLT_MAX
-// left of / below the mesh
-__device__ float bilinear(const LayerDev &m, const float *v, float xq, float yq) {
-  const float x0 = m.x0, x1 = __fadd_rn(m.x0, m.dx);
-  const float y0 = m.y0, y1 = __fadd_rn(m.y0, m.dy);
-  const int ix = (int)__fdiv_rn(__fsub_rn(xq, x0), __fsub_rn(x1, x0));
-  const int iy = (int)__fdiv_rn(__fsub_rn(yq, y0), __fsub_rn(y1, y0));
-  // (the reference checks only the lower side here; its callers keep points inside the mesh,
-  // and beyond the upper side there is nothing to read)
-  if (ix < 0 || iy < 0 || ix > m.nx - 1 || iy > m.ny - 1) return FLT_MAX;
-  const int indx = iy * m.nx + ix;
-  if (ix == m.nx - 1 || iy == m.ny - 1) return v[indx];
-  const float xa = __fadd_rn(m.x0, __fmul_rn(m.dx, (float)ix)), xb = __fadd_rn(m.x0, __fmul_rn(m.dx, (float)(ix + 1)));
-  const float ya = __fadd_rn(m.y0, __fmul_rn(m.dy, (float)iy)), yb = __fadd_rn(m.y0, __fmul_rn(m.dy, (float)(iy + 1)));
-  const float area = __fmul_rn(__fsub_rn(xb, xa), __fsub_rn(yb, ya));
-  float vq = __fmul_rn(__fmul_rn(v[indx], __fsub_rn(xb, xq)), __fsub_rn(yb, yq));
-  vq = __fadd_rn(vq, __fmul_rn(__fmul_rn(v[indx + 1], __fsub_rn(xq, xa)), __fsub_rn(yb, yq)));
-  vq = __fadd_rn(vq, __fmul_rn(__fmul_rn(v[indx + m.nx], __fsub_rn(xb, xq)), __fsub_rn(yq, ya)));
-  vq = __fadd_rn(vq, __fmul_rn(__fmul_rn(v[indx + 1 + m.nx], __fsub_rn(xq, xa)), __fsub_rn(yq, ya)));
-  return __fdiv_rn(vq, area);
-}
+// BilinearInterpolation (media_utility.cpp:325-360) on the uniform interface mesh: what depends on
+// the point only, computed once for the dozen arrays read at it, and the interpolation of one array
+// (FLT_MAX left of / below the mesh).
+struct MeshPoint {
+  int indx, nx;
+  bool out, edge;
+  float ax, bx, ay, by, area;  // xq - xa, xb - xq, yq - ya, yb - yq, (xb - xa)(yb - ya)
+  __device__ __forceinline__ MeshPoint(const LayerDev &m, float xq, float yq) {
+    const float x0 = m.x0, x1 = __fadd_rn(m.x0, m.dx);
+    const float y0 = m.y0, y1 = __fadd_rn(m.y0, m.dy);
+    const int ix = (int)__fdiv_rn(__fsub_rn(xq, x0), __fsub_rn(x1, x0));
+    const int iy = (int)__fdiv_rn(__fsub_rn(yq, y0), __fsub_rn(y1, y0));
+    nx = m.nx;
+    // (the reference checks only the lower side here; its callers keep points inside the mesh,
+    // and beyond the upper side there is nothing to read)
+    out = ix < 0 || iy < 0 || ix > m.nx - 1 || iy > m.ny - 1;
+    edge = ix == m.nx - 1 || iy == m.ny - 1;
+    indx = iy * m.nx + ix;
+    const float xa = __fadd_rn(m.x0, __fmul_rn(m.dx, (float)ix)), xb = __fadd_rn(m.x0, __fmul_rn(m.dx, (float)(ix + 1)));
+    const float ya = __fadd_rn(m.y0, __fmul_rn(m.dy, (float)iy)), yb = __fadd_rn(m.y0, __fmul_rn(m.dy, (float)(iy + 1)));
+    ax = __fsub_rn(xq, xa);
+    bx = __fsub_rn(xb, xq);
+    ay = __fsub_rn(yq, ya);
+    by = __fsub_rn(yb, yq);
+    area = __fmul_rn(__fsub_rn(xb, xa), __fsub_rn(yb, ya));
+  }
+  __device__ __forceinline__ float operator()(const float *v) const {
+    if (out) return FLT_MAX;
+    if (edge) return v[indx];
+    float vq = __fmul_rn(__fmul_rn(v[indx], bx), by);
+    vq = __fadd_rn(vq, __fmul_rn(__fmul_rn(v[indx + 1], ax), by));
+    vq = __fadd_rn(vq, __fmul_rn(__fmul_rn(v[indx + nx], bx), ay));
+    vq = __fadd_rn(vq, __fmul_rn(__fmul_rn(v[indx + 1 + nx], ax), ay));
+    return __fdiv_rn(vq, area);
+  }
+};
+
+__device__ float bilinear(const LayerDev &m, const float *v, float xq, float yq) { return MeshPoint(m, xq, yq)(v); }
 
 // findLastGreaterEqualIndex (media_utility.cpp:60-81): the last interface of the leading run at
 // or above `value`; -1 above the first interface
@@ -98,11 +117,9 @@ __device__ int first_ge(float value, const float *e, int n) {
 }
 
 // value + dz^pow * grad of layer mi at (x, y): the reference adds in double and stores float
-__device__ float layer_val(const LayerDev &m, int q, int mi, float x, float y, float dz) {
+__device__ __forceinline__ float layer_val(const LayerDev &m, int q, int mi, const MeshPoint &at, float dz) {
   const size_t sl = (size_t)m.nx * m.ny;
-  const float v = bilinear(m, m.p[3 * q] + mi * sl, x, y);
-  const float g = bilinear(m, m.p[3 * q + 1] + mi * sl, x, y);
-  const float pw = bilinear(m, m.p[3 * q + 2] + mi * sl, x, y);
+  const float v = at(m.p[3 * q] + mi * sl), g = at(m.p[3 * q + 1] + mi * sl), pw = at(m.p[3 * q + 2] + mi * sl);
   // the powers model files mostly use need no pow (a third of the averages' time in double)
   const double dp = pw == 1.f ? (double)dz : pw == 0.f ? 1.0 : pow((double)dz, (double)pw);
   return (float)__dadd_rn((double)v, __dmul_rn(dp, (double)g));
@@ -116,28 +133,29 @@ __device__ int point_value(const LayerDev &m, P3 a, float var[3]) {
   const float maxx = __fadd_rn(m.x0, __fmul_rn(m.dx, (float)(m.nx - 1)));
   const float maxy = __fadd_rn(m.y0, __fmul_rn(m.dy, (float)(m.ny - 1)));
   if (a.x < m.x0 || a.x > maxx || a.y < m.y0 || a.y > maxy) return 1;
+  const MeshPoint at(m, a.x, a.y);
   float e[kMaxInterfaces];
   const size_t sl = (size_t)m.nx * m.ny;
-  for (int n = 0; n < m.ni_; n++) e[n] = bilinear(m, m.elev + n * sl, a.x, a.y);
+  for (int n = 0; n < m.ni_; n++) e[n] = at(m.elev + n * sl);
   int mi = last_ge(a.z, e, m.ni_);
   if (mi == -1) {  // above the top interface: the top layer's values
     mi = last_ge(e[0], e, m.ni_);
-    for (int q = 0; q < 3; q++) var[q] = bilinear(m, m.p[3 * q] + mi * sl, a.x, a.y);
+    for (int q = 0; q < 3; q++) var[q] = at(m.p[3 * q] + mi * sl);
     return 0;
   }
   float dz = __fsub_rn(e[mi], a.z);
   // var[0] rho, var[1] vp, var[2] vs; the reference evaluates vp, vs, then rho
-  var[1] = layer_val(m, 1, mi, a.x, a.y, dz);
-  var[2] = layer_val(m, 2, mi, a.x, a.y, dz);
-  var[0] = layer_val(m, 0, mi, a.x, a.y, dz);
+  var[1] = layer_val(m, 1, mi, at, dz);
+  var[2] = layer_val(m, 2, mi, at, dz);
+  var[0] = layer_val(m, 0, mi, at, dz);
   if ((double)var[1] <= __dmul_rn((double)var[2], 1.4142135623730951)) return 2;
   if ((int)dz == 0) {  // on an interface (the reference's integer-abs test)
     const int mt = first_ge(a.z, e, m.ni_) - 1;
     if (mt >= 0) {
       dz = __fsub_rn(e[mt], a.z);
-      const float vpt = layer_val(m, 1, mt, a.x, a.y, dz);
-      const float vst = layer_val(m, 2, mt, a.x, a.y, dz);
-      const float rhot = layer_val(m, 0, mt, a.x, a.y, dz);
+      const float vpt = layer_val(m, 1, mt, at, dz);
+      const float vst = layer_val(m, 2, mt, at, dz);
+      const float rhot = layer_val(m, 0, mt, at, dz);
       // (a + b) / 2.0: a float sum, halved in double
       var[0] = (float)__ddiv_rn((double)__fadd_rn(var[0], rhot), 2.0);
       var[1] = (float)__ddiv_rn((double)__fadd_rn(var[1], vpt), 2.0);
@@ -161,22 +179,23 @@ __device__ int point_value_ac(const LayerDev &m, P3 a, float var[2]) {
   const float maxx = __fadd_rn(m.x0, __fmul_rn(m.dx, (float)(m.nx - 1)));
   const float maxy = __fadd_rn(m.y0, __fmul_rn(m.dy, (float)(m.ny - 1)));
   if (a.x < m.x0 || a.x > maxx || a.y < m.y0 || a.y > maxy) return 1;
+  const MeshPoint at(m, a.x, a.y);
   float e[kMaxInterfaces];
   const size_t sl = (size_t)m.nx * m.ny;
-  for (int n = 0; n < m.ni_; n++) e[n] = bilinear(m, m.elev + n * sl, a.x, a.y);
+  for (int n = 0; n < m.ni_; n++) e[n] = at(m.elev + n * sl);
   int mi = last_ge(a.z, e, m.ni_);
   if (mi == -1) {  // above the top interface: the top layer's values
     mi = last_ge(e[0], e, m.ni_);
-    for (int q = 0; q < 2; q++) var[q] = bilinear(m, m.p[3 * q] + mi * sl, a.x, a.y);
+    for (int q = 0; q < 2; q++) var[q] = at(m.p[3 * q] + mi * sl);
     return 0;
   }
   const float dz = __fsub_rn(e[mi], a.z);
-  var[0] = layer_val(m, 0, mi, a.x, a.y, dz);
-  var[1] = layer_val(m, 1, mi, a.x, a.y, dz);
+  var[0] = layer_val(m, 0, mi, at, dz);
+  var[1] = layer_val(m, 1, mi, at, dz);
   if ((int)dz == 0) {  // isEqual(dz, 0.0) with the integer abs()
     const int mt = first_ge(a.z, e, m.ni_) - 1;
     if (mt >= 0) {
-      const float rhot = layer_val(m, 0, mt, a.x, a.y, dz), vpt = layer_val(m, 1, mt, a.x, a.y, dz);
+      const float rhot = layer_val(m, 0, mt, at, dz), vpt = layer_val(m, 1, mt, at, dz);
       var[0] = (float)__ddiv_rn((double)__fadd_rn(var[0], rhot), 2.0);
       var[1] = (float)__ddiv_rn((double)__fadd_rn(var[1], vpt), 2.0);
     }
@@ -258,8 +277,9 @@ __global__ void k_mark(const __grid_constant__ LayerDev m, const __grid_constant
   const long long n = (long long)g.nx * g.ny * g.nz;
   const size_t sl = (size_t)m.nx * m.ny;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    const MeshPoint at(m, g.hx[t], g.hy[t]);
     float e[kMaxInterfaces];
-    for (int q = 0; q < m.ni_; q++) e[q] = bilinear(m, m.elev + q * sl, g.hx[t], g.hy[t]);
+    for (int q = 0; q < m.ni_; q++) e[q] = at(m.elev + q * sl);
     int mi = last_ge(g.hz[t], e, m.ni_);
     if (mi == -1) mi = last_ge(e[0], e, m.ni_);
     g.mat[t] = mi;
@@ -292,17 +312,21 @@ __global__ void k_mixed(const __grid_constant__ GridDev g, unsigned int *list, u
 // media_layer2model.cpp:1765-1960): rho arithmetically, kappa harmonically (har) or arithmetically
 // (ari); g.lam holds kappa.
 // One warp per point: the lanes evaluate 32 sub-points at a time (MeshSubdivide,
-// media_utility.cpp:421-448, in k, j, i order), then every lane adds the 32 terms in that order, so
-// the sums round as the reference's serial loop does. The evaluation (interface search, bilinear
-// parameters, double divisions) is what costs; one thread per grid point, 729 sub-points in turn,
-// left most lanes of a warp idle beside the few mixed points (22 ms on 192x176x96 with two
-// interfaces).
+// media_utility.cpp:421-448, in k, j, i order) and leave the terms in shared memory; three lanes, one
+// per accumulator, then add them in that order, so the sums round as the reference's serial loop does
+// (a float sum of two floats equals their double sum rounded to float, so one double chain serves rho
+// too). The evaluation (interface search, bilinear parameters, double divisions) is what costs.
+// 192x176x96 with two interfaces: 22 ms with one thread per grid point and its 729 sub-points in turn
+// (lanes idle beside the few mixed points), 4.2 ms so; a point per lane diverges in the search (25 ms).
 template <bool HAR, bool AC>
 __global__ void __launch_bounds__(128) k_media_avg(const __grid_constant__ LayerDev m, const __grid_constant__ GridDev g,
                                                    const unsigned int *list, const unsigned int *count) {
   constexpr int NS = kSub + 1, NSG = NS * NS * NS;
+  __shared__ double terms[4][3][32];
   const long long sl = g.nx, ss = (long long)g.nx * g.ny;
   const int lane = threadIdx.x & 31;
+  double(*term)[32] = terms[threadIdx.x >> 5];
+  const double *mine = term[lane < 3 ? lane : 0];
   const unsigned int n = *count;
   for (unsigned int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n; t += (gridDim.x * blockDim.x) >> 5) {
     const long long indx = list[t];
@@ -310,12 +334,15 @@ __global__ void __launch_bounds__(128) k_media_avg(const __grid_constant__ Layer
                             indx - 1 - sl,      indx - sl,      indx,      indx - 1};
     P3 M[8];
     for (int q = 0; q < 8; q++) M[q] = P3{g.hx[c[q]], g.hy[c[q]], g.hz[c[q]]};
-    float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f;  // rho, then kappa^-1 and mu^-1 (har) or lambda and mu (ari)
+    float acc = 0.f;  // lane 0: rho, lanes 1 and 2: kappa^-1 and mu^-1 (har) or lambda and mu (ari)
     int bad = 0;
-    auto lerp = [](P3 a, P3 b, int s) {  // a + (b - a) / ng * s, one rounding per step (Point3 operators)
-      return P3{__fadd_rn(a.x, __fmul_rn(__fdiv_rn(__fsub_rn(b.x, a.x), (float)kSub), (float)s)),
-                __fadd_rn(a.y, __fmul_rn(__fdiv_rn(__fsub_rn(b.y, a.y), (float)kSub), (float)s)),
-                __fadd_rn(a.z, __fmul_rn(__fdiv_rn(__fsub_rn(b.z, a.z), (float)kSub), (float)s))};
+    // a + (b - a) / ng * s, one rounding per step (Point3 operators); the division by 8 is exact as a
+    // product
+    auto lerp = [](P3 a, P3 b, int s) {
+      constexpr float inv = 1.0f / kSub;
+      return P3{__fadd_rn(a.x, __fmul_rn(__fmul_rn(__fsub_rn(b.x, a.x), inv), (float)s)),
+                __fadd_rn(a.y, __fmul_rn(__fmul_rn(__fsub_rn(b.y, a.y), inv), (float)s)),
+                __fadd_rn(a.z, __fmul_rn(__fmul_rn(__fsub_rn(b.z, a.z), inv), (float)s))};
     };
     for (int s0 = 0; s0 < NSG; s0 += 32) {
       const int sp = s0 + lane, ii = sp % NS, jj = sp / NS % NS, kk = sp / (NS * NS);
@@ -343,18 +370,18 @@ __global__ void __launch_bounds__(128) k_media_avg(const __grid_constant__ Layer
         }
       }
       bad |= rc;
-      const int cnt = min(32, NSG - s0);
-      for (int l = 0; l < cnt; l++) {
-        acc0 = __fadd_rn(acc0, __shfl_sync(0xffffffffu, f0, l));
-        if (HAR) {
-          acc1 = (float)__dadd_rn((double)acc1, __shfl_sync(0xffffffffu, d1, l));
-          if (!AC) acc2 = (float)__dadd_rn((double)acc2, __shfl_sync(0xffffffffu, d2, l));
-        } else {
-          acc1 = __fadd_rn(acc1, __shfl_sync(0xffffffffu, f1, l));
-          if (!AC) acc2 = __fadd_rn(acc2, __shfl_sync(0xffffffffu, f2, l));
-        }
+      term[0][lane] = (double)f0;
+      term[1][lane] = HAR ? d1 : (double)f1;
+      term[2][lane] = HAR ? d2 : (double)f2;
+      __syncwarp();
+      if (lane < 3) {
+        const int cnt = min(32, NSG - s0);
+        for (int l = 0; l < cnt; l++) acc = (float)__dadd_rn((double)acc, mine[l]);
       }
+      __syncwarp();
     }
+    const float acc0 = __shfl_sync(0xffffffffu, acc, 0), acc1 = __shfl_sync(0xffffffffu, acc, 1),
+                acc2 = __shfl_sync(0xffffffffu, acc, 2);
     bad = (int)__reduce_or_sync(0xffffffffu, (unsigned)bad);
     if (lane) continue;
     if (bad) { atomicOr(g.err, bad); continue; }  // the sums hold values of no meaning and are dropped
@@ -646,10 +673,11 @@ int layer_iso_family(int device, int ni, int nj, int nk, const float *coord, int
   const int nq = ac ? 6 : 9, nout = ac ? 2 : 3;
   const size_t nx = ni + 6, ny = nj + 6, nz = nk + 6, n = nx * ny * nz;
   const size_t msz = (size_t)num_interfaces * mnx * mny;
-  std::vector<void *> owned;
+  const bool avg = method != CGFD_MEDIA_LOC;
+  char *slab = nullptr;
   cudaStream_t st = nullptr;
   auto cleanup = [&] {
-    for (void *q : owned) cudaFree(q);
+    cudaFree(slab);
     if (st) cudaStreamDestroy(st);
   };
   auto fail = [&](cudaError_t e, const char *what) {
@@ -657,19 +685,25 @@ int layer_iso_family(int device, int ni, int nj, int nk, const float *coord, int
     set_last_error(std::string(what) + ": " + cudaGetErrorString(e));
     return e == cudaErrorMemoryAllocation ? CGFD_ERR_NOMEM : CGFD_ERR_CUDA;
   };
-  auto dalloc = [&](size_t bytes, void **out) {
-    cudaError_t e = cudaMalloc(out, bytes);
-    if (e == cudaSuccess) owned.push_back(*out);
-    return e;
-  };
   cudaError_t e = cudaSetDevice(device);
   if (e != cudaSuccess) return fail(e, "cudaSetDevice");
   if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "cudaStreamCreate");
+  // one allocation for the model, the coordinates, the result, and for the averages the half grid with
+  // its layer numbers (an allocation each, and its release, took milliseconds a call)
+  size_t used = 0;
+  auto carve = [&](size_t floats) {
+    const size_t at = used;
+    used += (floats * sizeof(float) + 255) / 256 * 256;
+    return at;
+  };
+  const size_t o_model = carve((1 + nq) * msz), o_coord = carve(3 * n), o_out = carve((size_t)nout * n), o_err = carve(1);
+  const size_t o_half = carve(avg ? 3 * n : 0), o_mat = carve(avg ? n : 0);
+  if ((e = cudaMalloc((void **)&slab, used)) != cudaSuccess) return fail(e, "cudaMalloc");
+  auto floats = [&](size_t at) { return reinterpret_cast<float *>(slab + at); };
   LayerDev m{};
   m.ni_ = num_interfaces; m.nx = mnx; m.ny = mny;
   m.x0 = x0; m.y0 = y0; m.dx = dx; m.dy = dy;
-  float *dm = nullptr;
-  if ((e = dalloc((1 + nq) * msz * sizeof(float), (void **)&dm)) != cudaSuccess) return fail(e, "cudaMalloc");
+  float *dm = floats(o_model);
   if ((e = cudaMemcpyAsync(dm, elevation, msz * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return fail(e, "cudaMemcpy");
   m.elev = dm;
@@ -680,11 +714,8 @@ int layer_iso_family(int device, int ni, int nj, int nk, const float *coord, int
   }
   GridDev g;
   g.nx = (int)nx; g.ny = (int)ny; g.nz = (int)nz;
-  float *dc = nullptr, *dout = nullptr;
-  int *derr = nullptr;
-  if ((e = dalloc(3 * n * sizeof(float), (void **)&dc)) != cudaSuccess) return fail(e, "cudaMalloc");
-  if ((e = dalloc((size_t)nout * n * sizeof(float), (void **)&dout)) != cudaSuccess) return fail(e, "cudaMalloc");
-  if ((e = dalloc(sizeof(int), (void **)&derr)) != cudaSuccess) return fail(e, "cudaMalloc");
+  float *dc = floats(o_coord), *dout = floats(o_out);
+  int *derr = reinterpret_cast<int *>(slab + o_err);
   if ((e = cudaMemcpyAsync(dc, coord, 3 * n * sizeof(float), cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return fail(e, "cudaMemcpy");
   cudaMemsetAsync(derr, 0, sizeof(int), st);
@@ -696,13 +727,10 @@ int layer_iso_family(int device, int ni, int nj, int nk, const float *coord, int
   g.mat = nullptr;
   if (ac) k_media_loc<true><<<148 * 8, 256, 0, st>>>(m, g);
   else k_media_loc<false><<<148 * 8, 256, 0, st>>>(m, g);
-  if (method != CGFD_MEDIA_LOC) {
-    float *dh = nullptr;
-    int *dmat = nullptr;
-    if ((e = dalloc(3 * n * sizeof(float), (void **)&dh)) != cudaSuccess) return fail(e, "cudaMalloc");
-    if ((e = dalloc(n * sizeof(int), (void **)&dmat)) != cudaSuccess) return fail(e, "cudaMalloc");
+  if (avg) {
+    float *dh = floats(o_half);
     g.hx = dh; g.hy = dh + n; g.hz = dh + 2 * n;
-    g.mat = dmat;
+    g.mat = reinterpret_cast<int *>(slab + o_mat);
     k_half_grid<<<148 * 8, 256, 0, st>>>(g);
     k_mark<<<148 * 8, 256, 0, st>>>(m, g);
     // the mixed points, their count last, where the coordinates were (3 n floats, not read any more)
@@ -721,9 +749,20 @@ int layer_iso_family(int device, int ni, int nj, int nk, const float *coord, int
   int herr = 0;
   if ((e = cudaMemcpyAsync(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess)
     return fail(e, "cudaMemcpy");
-  if ((e = cudaMemcpyAsync(medium, dout, (size_t)nout * n * sizeof(float), cudaMemcpyDeviceToHost, st)) !=
-      cudaSuccess)
+  const size_t bytes = (size_t)nout * n * sizeof(float);
+  if (bytes >= PinnedStager::kMinBytes) {
+    try {
+      PinnedStager &ps = PinnedStager::for_device(device);
+      std::lock_guard<std::mutex> lk(ps.mutex());
+      ps.copy_out(medium, dout, bytes, st);
+    } catch (const Error &x) {
+      cleanup();
+      set_last_error(x.what());
+      return x.code;
+    }
+  } else if ((e = cudaMemcpyAsync(medium, dout, bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
     return fail(e, "cudaMemcpy");
+  }
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return fail(e, "cudaStreamSynchronize");
   cleanup();
   if (herr) {
