@@ -463,9 +463,14 @@ __device__ __forceinline__ void ac_tile(const StageP &p, const TmaP &tm, const i
           const FaceP &fc = p.face[fi];
           // (an index into the register arrays by fc.axis would put them in local memory for every
           // cell, PML or not)
-          if (fc.axis == 0) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[0], dv[0], dp[0], hc);
-          else if (fc.axis == 1) ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[1], dv[1], dp[1], hc);
-          else ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mt[2], dv[2], dp[2], hc);
+          float mrow[3], vrow[3];
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            mrow[c] = fc.axis == 0 ? mt[0][c] : fc.axis == 1 ? mt[1][c] : mt[2][c];
+            vrow[c] = fc.axis == 0 ? dv[0][c] : fc.axis == 1 ? dv[1][c] : dv[2][c];
+          }
+          const float prow = fc.axis == 0 ? dp[0] : fc.axis == 1 ? dp[1] : dp[2];
+          ac_pml_face(p, fc, i, j, k, shot, slw, kappa, mrow, vrow, prow, hc);
         }
 #pragma unroll
         for (int c = 0; c < kAcF; c++) h[c] += hc[c];

@@ -345,7 +345,7 @@ struct cgfd_problem {
     if (med == cgfd::MED_AC) return fp64 ? 1 : cgfd::ac_tma_resident();
     if (tma64) return cgfd::tma64_resident(med);
     if (fp64) return 1;
-    if (vis) return vis_tma ? cgfd::tma_blocks_per_sm(med, shape) : 2;
+    if (vis) return vis_tma ? cgfd::vis_bulk_resident() : 2;
     return cgfd::tma_resident(med, coef_type, wave16, shape);
   }
 
@@ -1389,12 +1389,13 @@ std::vector<std::pair<int, int>> z_ranges(const cgfd_problem *p, int nzc) {
 // takes chunks of about 12 planes: a chunk's 3-plane prologue comes from L2, and short chunks keep
 // the resident blocks on neighbouring planes. A grid with fewer blocks than kFew resident sets at 12
 // planes is bound by the time its last set takes, so it takes the chunk length c that minimises
-// ceil(blocks / resident) (longest chunk + 3): sets of blocks, each as long as its longest block with
-// its prologue. us per step, 12 planes against the rule's choice: 64x64x64 235 against 122 (4
-// planes), 100x100x60 312 against 283 (5 planes); 5 shots of 141x118x77, 6.5 sets, 1780 at 12 planes
+// ceil(blocks / resident) (longest chunk + prologue): sets of blocks, each as long as its longest
+// block with its prologue. us per step, 12 planes against the rule's choice: 64x64x64 235 against 122 (4
+// planes), 100x100x60 312 against 283 (5 planes), 180x180x80 (3.2 sets) 677 against 652 (6 planes); 5 shots of 141x118x77, 6.5 sets, 1780 at 12 planes
 // and 1785-1830 at 4-8.
 int default_chunk(const cgfd_problem *p) {
-  constexpr int kFew = 3, kPrologue = 3;
+  constexpr int kFew = 4;
+  const int prologue = p->vis ? 1 : 3;  // in planes (a plane of visco-elastic cells costs about three elastic ones)
   if (p->nbulk < 1) return 1;
   int nsm = 148;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
@@ -1423,7 +1424,7 @@ int default_chunk(const cgfd_problem *p) {
   long long best_cost = LLONG_MAX;
   for (int c = 12; c >= 3; c--) {
     const long long blocks = columns * chunks(c, longest);
-    const long long cost = (blocks + resident - 1) / resident * (longest + kPrologue);
+    const long long cost = (blocks + resident - 1) / resident * (longest + prologue);
     if (cost < best_cost) { best_cost = cost; best = c; }
   }
   return best;

@@ -73,7 +73,7 @@ struct BulkSmem {
   // resident blocks the registers are budgeted for: a fourth 32x4 block of iso tiles (57 KB each)
   // fits beside three at 128 registers per thread, and is worth 3-5% over three at 168
   static constexpr int BOUND = MED == MED_ISO && MINB == 3 && 4 * (BYTES + 1024) <= 228 * 1024 ? 4 : MINB;
-  static constexpr bool ONE_ROUND = sizeof(real_of<TC>) == 4 && BOUND * CELLS * 168 <= 65536;
+  static constexpr bool ONE_ROUND = sizeof(real_of<TC>) == 4;  // AuxPoint: 114 -> 128 registers (iso)
   static_assert(NW + 2 <= 8, "mbarrier area");
   static_assert(COEF_BYTES % 128 == 0, "w_pre/w_end boxes must stay 128-byte aligned");
   static_assert(MINB == 1 || MINB * (BYTES + 1024) <= 228 * 1024, "MINB blocks must fit one SM's shared memory");
@@ -263,15 +263,28 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
           if (!(tmask >> fi & 1)) continue;
           const FacePT<R> &fc = p.face[fi];
           R d[9];
-          if (fc.axis == 0) {
+          auto face = [&](const R mrow[3]) {
+            pml_face<MED, (S::ONE_ROUND && VIS <= 2)>(p, fc, i, j, k, md, slw, mrow, d, d + 3, nullptr, nullptr, h, shot);
+          };
+          if constexpr (sizeof(R) == 4) {
+            // one copy of the face code for the three axes: it frees 10-16 registers, which hold what
+            // the auxiliaries' RK combine reads (in double the selected row costs more than that)
+            R mrow[3];
+            if (fc.axis == 0) deriv_x(d);
+            else if (fc.axis == 1) deriv_y(d);
+            else deriv_z(d);
+#pragma unroll
+            for (int c = 0; c < 3; c++) mrow[c] = fc.axis == 0 ? mt[0][c] : fc.axis == 1 ? mt[1][c] : mt[2][c];
+            face(mrow);
+          } else if (fc.axis == 0) {
             deriv_x(d);
-            pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[0], d, d + 3, nullptr, nullptr, h, shot);
+            face(mt[0]);
           } else if (fc.axis == 1) {
             deriv_y(d);
-            pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[1], d, d + 3, nullptr, nullptr, h, shot);
+            face(mt[1]);
           } else {
             deriv_z(d);
-            pml_face<MED, S::ONE_ROUND>(p, fc, i, j, k, md, slw, mt[2], d, d + 3, nullptr, nullptr, h, shot);
+            face(mt[2]);
           }
         }
       }

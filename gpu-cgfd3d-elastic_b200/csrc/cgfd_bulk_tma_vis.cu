@@ -1,13 +1,14 @@
 // cgfd_bulk_tma_vis.cu -- the bulk RK-stage kernel's visco-elastic form: the iso stage with the
 // attenuation of each point between its right-hand side and its RK combine, so that the 9-field
 // right-hand side never reaches memory. Bound by the memory variables' own traffic (18 NM floats
-// read and 12 NM written per cell at stages 1-2 beside the iso stage's 45): three blocks per SM of
-// 32x4 columns leave 168 registers for the next mechanism's loads.
+// read and 12 NM written per cell at stages 1-2 beside the iso stage's 45), and by latency: four blocks
+// per SM of 32x4 columns at 128 registers run 160x160x80 with 3 mechanisms in 1199 us per step, three
+// at 168 in 1244.
 #include "cgfd_bulk_tma.cuh"
 
 namespace cgfd {
 
-constexpr int kVisTY = 4, kVisBlocks = 3;
+constexpr int kVisTY = 4, kVisBlocks = 4;
 
 template <int DX, int DY, int DZ, int NM>
 __global__ void __launch_bounds__(TX *kVisTY, kVisBlocks)
@@ -39,6 +40,7 @@ static cudaError_t for_each_dir(int code, const StageP *p, const TmaP *tm, const
 }
 
 int vis_bulk_max_mechanisms() { return 4; }
+int vis_bulk_resident() { return kVisBlocks; }
 
 static cudaError_t dispatch(int nmax, const StageP *p, const TmaP *tm, const VisP *v, const BulkTiles *t,
                             cudaStream_t st) {

@@ -320,10 +320,10 @@ __device__ __forceinline__ R *face_aux(const FacePT<R> &f, int i, int j, int k, 
 }
 
 // The N auxiliaries of one point and their RK combine. ONE_ROUND: what the combine reads is loaded
-// together with the stage input, one round trip to memory instead of two, for kernels with the
-// registers to hold 3 N values across the right-hand side (168 per thread: 21-Cij tiles 1345 -> 1244 us
-// per step on 203x187x121, against 1316 in two rounds); at 128 registers it spills and loses more
-// than it gains (iso tiles on 480x480x240: 10.0 ms per step before, 9.74 in two rounds, 11.1 in one).
+// together with the stage input, one round trip to memory instead of two, for kernels whose
+// registers hold 3 N values across the right-hand side without spilling. us per step, two rounds
+// against one: iso 480x480x240 9980 / 9899, 5 shots of 141x118x77 1668 / 1621, 21-Cij 203x187x121
+// 1316 / 1236; where it spills it loses more than it gains (480x480x240, 200 bytes: 11100).
 template <int N, bool ONE_ROUND, typename R>
 struct AuxPoint {
   R *a;

@@ -180,6 +180,7 @@ int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, c
 // up to vis_bulk_max_mechanisms() mechanisms (media with more run the direct-load kernel and the
 // separate attenuation pass).
 int vis_bulk_max_mechanisms();
+int vis_bulk_resident();  // blocks per SM
 cudaError_t tma_prepare_vis(int nmax);
 int launch_stage_bulk_vis(const StageP &p, const TmaP &tm, const VisP &v, const BulkTiles &t, cudaStream_t st);
 // FP16 stage levels: per-step scale from the last step's max |w| and the step's source bound
