@@ -16,15 +16,18 @@ namespace cgfd {
 template <int NM>
 __device__ __forceinline__ void vis_atten(const VisP &q, int stage, long long id, float lam, float mu, float h[9]) {
   const long long sf = q.sf;
-  // isotropic compliance; the diagonal in double, as the reference's double literals make it
+  // isotropic compliance, in double as the reference's double literals make it; one division for the
+  // six quotients by 2 mu (each within 2^-52 before it is rounded to float)
   const float tr = (h[3] + h[4] + h[5]) / (3.f * lam + 2.f * mu);
+  const double inv2mu = 1.0 / (double)(2.f * mu);
+  constexpr double third = 1.0 / 3.0;
   float ev[6];
-  ev[0] = (float)(((2.0 * h[3] - h[4] - h[5]) / (double)(2.f * mu) + tr) / 3.0);
-  ev[1] = (float)(((2.0 * h[4] - h[3] - h[5]) / (double)(2.f * mu) + tr) / 3.0);
-  ev[2] = (float)(((2.0 * h[5] - h[3] - h[4]) / (double)(2.f * mu) + tr) / 3.0);
-  ev[3] = (float)((double)(h[6] / mu) * 0.5);
-  ev[4] = (float)((double)(h[7] / mu) * 0.5);
-  ev[5] = (float)((double)(h[8] / mu) * 0.5);
+  ev[0] = (float)(((2.0 * h[3] - h[4] - h[5]) * inv2mu + tr) * third);
+  ev[1] = (float)(((2.0 * h[4] - h[3] - h[5]) * inv2mu + tr) * third);
+  ev[2] = (float)(((2.0 * h[5] - h[3] - h[4]) * inv2mu + tr) * third);
+  ev[3] = (float)((double)h[6] * inv2mu);
+  ev[4] = (float)((double)h[7] * inv2mu);
+  ev[5] = (float)((double)h[8] * inv2mu);
   float sl = 0.f, sm[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const bool need_pre = stage == 1 || stage == 2, need_end = stage >= 1;
   struct Mech { float ylam, ymu, j[6], pre[6], end[6]; };
