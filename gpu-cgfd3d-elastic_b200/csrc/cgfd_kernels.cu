@@ -207,7 +207,9 @@ __device__ __forceinline__ void ld5(int dir, const WaveIn<TW> &cur, int f, long 
 }
 
 // Surface slab: one thread per cell of the top NSURF planes; a block holds the NSURF planes of
-// 32 x 2 columns, so that the z-stencil loads of one column hit in the SM's L1. WP is the wave
+// 32 columns of one row, so that the z-stencil loads of one column hit in the SM's L1 and a block's
+// 16 k registers are those of the one bulk block whose place it takes (with 32 x 2 columns two had to
+// retire on one SM: 64x64x64 112 -> 107 us per step, 480x480x240 9848 -> 9804). WP is the wave
 // policy of the bulk kernel (0 FP32 stage levels; 1 FP32 input, FP16 output; 2 FP16 input and
 // output). The kernel is latency-bound on its many cached loads: registers are capped at 128 so
 // that 16 warps share each SM (a few spills are cheaper than 8 warps).
@@ -236,25 +238,28 @@ __global__ void __launch_bounds__(128) k_timg_flux(const __grid_constant__ Stage
     const int tr[3][3] = {{3, 8, 7}, {8, 4, 6}, {7, 6, 5}};
     const R jc = __ldg(p.jac + q);
     R *out = p.flux + shot * per_shot + (long long)pl * plane + (long long)jj * nxe + ii;
+    // the slab's x and y operators run on its image planes only (the top 4 of forward, 2 of backward z
+    // operators); the z operator reaches every plane
+    const bool xy = pl >= (p.dir[2] ? 1 : 3);
 #pragma unroll
     for (int c = 0; c < 3; c++) {
       const R t1 = cur(tr[c][0], q), t2 = cur(tr[c][1], q), t3 = cur(tr[c][2], q);
 #pragma unroll
       for (int a = 0; a < 3; a++)
-        out[(3 * c + a) * kFluxPlanes * plane] = jc * (cv(3 * a, q) * t1 + cv(3 * a + 1, q) * t2 + cv(3 * a + 2, q) * t3);
+        if (a == 2 || xy) out[(3 * c + a) * kFluxPlanes * plane] = jc * (cv(3 * a, q) * t1 + cv(3 * a + 1, q) * t2 + cv(3 * a + 2, q) * t3);
     }
   }
 }
 
 template <int MED, typename TC, int WP, int DX, int DY, int DZ>
-__global__ void __launch_bounds__(32 * 2 * NSURF, 2) k_stage_surface(const __grid_constant__ StagePT<real_of<TC>> p) {
+__global__ void __launch_bounds__(32 * NSURF, 4) k_stage_surface(const __grid_constant__ StagePT<real_of<TC>> p) {
   constexpr int DIR[3] = {DX, DY, DZ};
   using R = real_of<TC>;  // double in the FP64 build (TC double, WP 0), float otherwise
   using TW = typename std::conditional<WP == 2, __half, R>::type;
   using TT = typename std::conditional<WP >= 1, __half, R>::type;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= p.ni || j >= p.nj) return;
+  const int nbx = (p.ni + 31) / 32, j = blockIdx.x / nbx;
+  const int i = (blockIdx.x - j * nbx) * 32 + threadIdx.x;
+  if (i >= p.ni) return;
   const long long sf = p.sf;
   const int shot = blockIdx.z;
   const long long woff = (long long)shot * 9 * sf;
@@ -757,8 +762,8 @@ int launch_timg_flux64(const StagePT<double> &p, cudaStream_t st) {
 
 int launch_stage_surface(int med, int coef_type, int wave16, const StageP &p, cudaStream_t st) {
   if (p.nbulk >= p.nk) return 0;
-  dim3 block(32, 2, NSURF);
-  dim3 grid((p.ni + 31) / 32, (p.nj + 1) / 2, p.nshot);
+  dim3 block(32, 1, NSURF);
+  dim3 grid((unsigned)((p.ni + 31) / 32) * p.nj, 1, p.nshot);
   if (wave16) {
     if (p.stage == 0) launch_surface_tc<uint16_t, 1>(med, p, grid, block, st);
     else launch_surface_tc<uint16_t, 2>(med, p, grid, block, st);
@@ -771,8 +776,8 @@ int launch_stage_surface(int med, int coef_type, int wave16, const StageP &p, cu
 
 int launch_stage_surface64(int med, const StagePT<double> &p, cudaStream_t st) {
   if (p.nbulk >= p.nk) return 0;
-  dim3 block(32, 2, NSURF);
-  dim3 grid((p.ni + 31) / 32, (p.nj + 1) / 2, p.nshot);
+  dim3 block(32, 1, NSURF);
+  dim3 grid((unsigned)((p.ni + 31) / 32) * p.nj, 1, p.nshot);
   launch_surface_tc<double, 0>(med, p, grid, block, st);
   return 1;
 }
