@@ -318,7 +318,7 @@ __device__ __forceinline__ void ac_tile(const StageP &p, const TmaP &tm, const i
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + S::OFF_BAR);  // NW wave, then 2 cpe
 
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int bx = tl.x & kTileBxMask, by = tl.y, shot = tl.x >> 16;
+  const int bx = tl.x & kTileBxMask, by = tl.y, shot = tl.x >> kTileShotShift & kTileShotMask;
   const int kb = tl.z, ke = tl.w;
   if (kb >= ke) return;
   const int n = ke - kb;

@@ -188,6 +188,9 @@ struct cgfd_problem {
 
   cgfd::SrcHost src;
   bool src_top = false;  // a source's smoothing points reach the top plane
+  bool src_bulk = false;  // at most kTileSources sources, no smoothing point in the surface slab
+  struct Box { int lo[3], hi[3]; };
+  std::vector<Box> src_box;  // of each source's smoothing points
   std::vector<int> src_shot;
   int *d_it_begin = nullptr, *d_ext_num = nullptr, *d_src_shot = nullptr;
   long long *d_ext_idx = nullptr;
@@ -206,7 +209,7 @@ struct cgfd_problem {
   int *d_slice_idx = nullptr;
   float *d_slices = nullptr;
 
-  int *d_it = nullptr, *d_flag = nullptr;
+  int *d_it = nullptr, *d_flag = nullptr;  // d_it[parity]: the step, for the steps of that parity
   int it = 0;
   // free-surface peak ground motion [nshot][15][nj][ni] and displacement [nshot][3][nj][ni]
   float *d_pg = nullptr, *d_dis = nullptr;
@@ -349,6 +352,24 @@ struct cgfd_problem {
     return cgfd::tma_resident(med, coef_type, wave16, shape);
   }
 
+  // Sources whose smoothing points all lie in the bulk planes, few enough for a tile to look through,
+  // are injected by the tiles of the TMA stage kernels (kTileSource); others by the source kernel.
+  bool src_in_tiles() const { return src_bulk && (use_tma || vis_tma || tma64); }
+
+  template <typename R>
+  cgfd::SrcPT<R> source_params(const cgfd::StagePT<R> &p, int step) const {
+    cgfd::SrcPT<R> q;
+    memset(&q, 0, sizeof(q));
+    q.nsrc = src.nsrc; q.max_ext = src.max_ext; q.max_nt = src.max_nt;
+    q.force = src.force; q.moment = src.moment; q.stage = p.stage;
+    q.ca = p.ca; q.cb = p.cb;
+    q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
+    q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
+    q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it + (step & 1);
+    q.wave16 = wave16; q.wsc = d_wsc; q.amax = d_amax;
+    return q;
+  }
+
   // tensor maps of one stage: the stage input, w_pre, w_end, coefficients
   cgfd::TmaP stage_maps(int step, int s) const {
     cgfd::TmaP tm;
@@ -369,7 +390,7 @@ struct cgfd_problem {
     if (nline > 0) {
       cgfd::RecvPT<R> r;
       r.nsta = nline; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_line_idx8; r.w8 = d_line_w8;
-      r.pre = rptr<R>(wbuf[step & 1]); r.sf = sf; r.seis = d_line_seis; r.d_it = d_it; r.d_flag = d_flag;
+      r.pre = rptr<R>(wbuf[step & 1]); r.sf = sf; r.seis = d_line_seis; r.d_it = d_it + (step & 1); r.d_flag = d_flag;
       n += timed(6, [&] { return cgfd::launch_recv(r, st); });
     }
     if (slice_per_shot > 0) {
@@ -378,7 +399,7 @@ struct cgfd_problem {
       q.sx = sx; q.sz = sz; q.sf = sf; q.off0 = off0;
       q.pre = rptr<R>(wbuf[step & 1]);
       q.nxs = nslx; q.nys = nsly; q.nzs = nslz; q.idx = d_slice_idx;
-      q.ring = d_slices; q.ring_steps = slice_ring; q.per_shot = slice_per_shot; q.d_it = d_it;
+      q.ring = d_slices; q.ring_steps = slice_ring; q.per_shot = slice_per_shot; q.d_it = d_it + (step & 1);
       n += timed(6, [&] { return cgfd::launch_slices(q, st); });
     }
     return n;
@@ -397,7 +418,7 @@ struct cgfd_problem {
       if (rec.n > 0) {
         cgfd::RecvPT<double> r;
         r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-        r.pre = rptr<double>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+        r.pre = rptr<double>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it + (step & 1); r.d_flag = d_flag;
         k += timed(6, [&] { return cgfd::launch_recv(r, s2); });
       }
       return k + enqueue_outputs<double>(step, s2);
@@ -413,14 +434,14 @@ struct cgfd_problem {
     if (!fork) n += sample(st);
     for (int s = 0; s < 4; s++) {
       const cgfd::StagePT<double> p = stage_params_t<double>(step, s);
-      const bool beside = fork && (free_top || s == 0 || s == 3);
+      const bool beside = fork && (free_top || s == 0);
       if (beside) {
         CK(cudaEventRecord(ev_fork, st));
         CK(cudaStreamWaitEvent(side, ev_fork, 0));
       }
       if (tma64) {
         const cgfd::TmaP tm = stage_maps(step, s);
-        n += timed(s, [&] { return cgfd::launch_stage_bulk_tma64(med, p, tm, p.dir[2] ? tiles_dn : tiles, st); });
+        n += timed(s, [&] { return cgfd::launch_stage_bulk_tma64(med, p, tm, source_params(p, step), p.dir[2] ? tiles_dn : tiles, st); });
       } else {
         n += timed(s, [&] { return cgfd::launch_stage_bulk(med, p, nzc, st); });
       }
@@ -428,27 +449,15 @@ struct cgfd_problem {
       n += timed(4, [&] { return cgfd::launch_timg_flux64(p, top) + cgfd::launch_stage_surface64(med, p, top); });
       if (beside) {
         if (s == 0) n += sample(side);
-        if (s == 3) {
-          if (early_peak) n += peak(side);
-          n += cgfd::launch_advance(d_it, side);
-        }
+        if (s == 0) n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), side);
+        if (s == 3 && early_peak) n += peak(side);
         CK(cudaEventRecord(ev_join, side));
         CK(cudaStreamWaitEvent(st, ev_join, 0));
       }
-      if (src.nsrc > 0) {
-        cgfd::SrcPT<double> q;
-        memset(&q, 0, sizeof(q));
-        q.nsrc = src.nsrc; q.max_ext = src.max_ext; q.max_nt = src.max_nt;
-        q.force = src.force; q.moment = src.moment; q.stage = s;
-        q.ca = p.ca; q.cb = p.cb;
-        q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
-        q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it; q.it_ahead = beside && s == 3;
-        n += timed(5, [&] { return cgfd::launch_source(q, st); });
-      }
+      if (src.nsrc > 0 && !src_in_tiles()) n += timed(5, [&] { return cgfd::launch_source(source_params(p, step), st); });
     }
     if (free_top && !early_peak) n += peak(st);
-    if (!fork) n += cgfd::launch_advance(d_it, st);
+    if (!fork) n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), st);
     return n;
   }
 
@@ -468,7 +477,7 @@ struct cgfd_problem {
       if (rec.n > 0) {
         cgfd::RecvPT<float> r;
         r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-        r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+        r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it + (step & 1); r.d_flag = d_flag;
         k += timed(6, [&] { return cgfd::launch_recv(r, s2); });
       }
       return k + enqueue_outputs<float>(step, s2);
@@ -488,14 +497,14 @@ struct cgfd_problem {
       v.coef = coef; v.y = d_y;
       for (int m = 0; m < nmax; m++) v.wl[m] = wl[m];
       v.ca = p.ca; v.cb = p.cb; v.err = d_flag;
-      const bool beside = fork && (free_top || s == 0 || s == 3);
+      const bool beside = fork && (free_top || s == 0);
       if (beside) {
         CK(cudaEventRecord(ev_fork, st));
         CK(cudaStreamWaitEvent(side, ev_fork, 0));
       }
       if (vis_tma) {
         const cgfd::TmaP tm = stage_maps(step, s);
-        n += timed(s, [&] { return cgfd::launch_stage_bulk_vis(p, tm, v, p.dir[2] ? tiles_dn : tiles, st); });
+        n += timed(s, [&] { return cgfd::launch_stage_bulk_vis(p, tm, v, source_params(p, step), p.dir[2] ? tiles_dn : tiles, st); });
       }
       p.rhs = d_rhs;
       if (!vis_tma) n += timed(s, [&] { return cgfd::launch_stage_bulk(cgfd::MED_ISO, p, nzc, st); });
@@ -508,21 +517,11 @@ struct cgfd_problem {
       n += timed(s, [&] { return cgfd::launch_vis_atten(v, top); });
       if (beside) {
         if (s == 0) n += sample(side);
-        if (s == 3) n += cgfd::launch_advance(d_it, side);
+        if (s == 0) n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), side);
         CK(cudaEventRecord(ev_join, side));
         CK(cudaStreamWaitEvent(st, ev_join, 0));
       }
-      if (src.nsrc > 0) {
-        cgfd::SrcPT<float> q;
-        memset(&q, 0, sizeof(q));
-        q.nsrc = src.nsrc; q.max_ext = src.max_ext; q.max_nt = src.max_nt;
-        q.force = src.force; q.moment = src.moment; q.stage = s;
-        q.ca = p.ca; q.cb = p.cb;
-        q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
-        q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it; q.it_ahead = beside && s == 3;
-        n += timed(5, [&] { return cgfd::launch_source(q, st); });
-      }
+      if (src.nsrc > 0 && !src_in_tiles()) n += timed(5, [&] { return cgfd::launch_source(source_params(p, step), st); });
     }
     if (free_top) {
       cgfd::VisFreeP f;
@@ -536,7 +535,7 @@ struct cgfd_problem {
       q.pg = d_pg; q.dis = d_dis; q.dt = dt;
       n += cgfd::launch_peak_motion(q, st);
     }
-    if (!fork) n += cgfd::launch_advance(d_it, st);
+    if (!fork) n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), st);
     return n;
   }
 
@@ -550,7 +549,7 @@ struct cgfd_problem {
     if (rec.n > 0) {
       cgfd::RecvPT<R> r;
       r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-      r.pre = rptr<R>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+      r.pre = rptr<R>(wbuf[step & 1]); r.sf = sf; r.seis = d_seis; r.d_it = d_it + (step & 1); r.d_flag = d_flag;
       n += timed(6, [&] { return cgfd::launch_recv(r, st); });
     }
     n += enqueue_outputs<R>(step, st);
@@ -562,17 +561,7 @@ struct cgfd_problem {
           if (ac_tma) return k + cgfd::launch_stage_ac_tma(p, stage_maps(step, s), p.dir[2] ? tiles_dn : tiles, st);
         return k + cgfd::launch_stage_ac(p, nzc, st);
       });
-      if (src.nsrc > 0) {
-        cgfd::SrcPT<R> q;
-        memset(&q, 0, sizeof(q));
-        q.nsrc = src.nsrc; q.max_ext = src.max_ext; q.max_nt = src.max_nt;
-        q.force = src.force; q.moment = src.moment; q.stage = s;
-        q.ca = p.ca; q.cb = p.cb;
-        q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
-        q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it;
-        n += timed(5, [&] { return cgfd::launch_source(q, st); });
-      }
+      if (src.nsrc > 0 && !src_in_tiles()) n += timed(5, [&] { return cgfd::launch_source(source_params(p, step), st); });
     }
     if (free_top) {
       cgfd::PgPT<R> q;
@@ -582,7 +571,7 @@ struct cgfd_problem {
       q.pg = d_pg; q.dis = rptr<R>(d_dis); q.dt = dt;
       n += cgfd::launch_peak_motion(q, st);
     }
-    n += cgfd::launch_advance(d_it, st);
+    n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), st);
     return n;
   }
 
@@ -596,9 +585,10 @@ struct cgfd_problem {
     // do not depend on:
     //   every stage: the flux pass and the surface slab (latency-bound, top planes only: they
     //     write planes of the stage outputs that no bulk tile reads or writes in this stage);
-    //   stage 0: the station, line and slice samples (they read w_pre, which stage 0 leaves alone);
+    //   stage 0: the station, line and slice samples (they read w_pre, which stage 0 leaves alone) and
+    //     the next step's counter (steps of either parity read their own);
     //   stage 3: peak motion (top plane of w_end, complete after the slab unless a source reaches
-    //     that plane) and the step counter, which the stage's sources then read one ahead.
+    //     that plane).
     // On the main stream these small kernels took 17 us of every step (5% of a 100x100x60 step).
     const bool fork = use_tma && tiles.n > 0 && !timing;
     const bool early_peak = fork && free_top && !src_top;
@@ -607,7 +597,7 @@ struct cgfd_problem {
       if (rec.n > 0) {
         cgfd::RecvP r;
         r.nsta = rec.n; r.nshot = nshot; r.nt_total = nt_total; r.idx8 = d_idx8; r.w8 = d_w8;
-        r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it; r.d_flag = d_flag;
+        r.pre = wbuf[step & 1]; r.sf = sf; r.seis = d_seis; r.d_it = d_it + (step & 1); r.d_flag = d_flag;
         k += timed(6, [&] { return cgfd::launch_recv(r, s2); });
       }
       return k + enqueue_outputs<float>(step, s2);
@@ -622,10 +612,10 @@ struct cgfd_problem {
     };
     if (!fork) n += sample(st);
     if (wave16)
-      n += timed(7, [&] { return cgfd::launch_wave_scale(d_amax, d_srcb, d_it, nt_total, nshot, d_wsc, st); });
+      n += timed(7, [&] { return cgfd::launch_wave_scale(d_amax, d_srcb, d_it + (step & 1), nt_total, nshot, d_wsc, st); });
     for (int s = 0; s < 4; s++) {
       cgfd::StageP p = stage_params(step, s);
-      const bool beside = fork && (free_top || s == 0 || s == 3);
+      const bool beside = fork && (free_top || s == 0);
       if (beside) {
         CK(cudaEventRecord(ev_fork, st));
         CK(cudaStreamWaitEvent(side, ev_fork, 0));
@@ -633,7 +623,8 @@ struct cgfd_problem {
       if (use_tma) {
         const cgfd::TmaP tm = stage_maps(step, s);
         n += timed(s, [&] {
-          return cgfd::launch_stage_bulk_tma(med, coef_type, wave16, shape, p, tm, p.dir[2] ? tiles_dn : tiles, st);
+          return cgfd::launch_stage_bulk_tma(med, coef_type, wave16, shape, p, tm, source_params(p, step),
+                                             p.dir[2] ? tiles_dn : tiles, st);
         });
       } else {
         n += timed(s, [&] { return cgfd::launch_stage_bulk(med, p, nzc, st); });
@@ -645,28 +636,16 @@ struct cgfd_problem {
       });
       if (beside) {
         if (s == 0) n += sample(side);
-        if (s == 3) {
-          if (early_peak) n += peak(side);
-          n += cgfd::launch_advance(d_it, side);
-        }
+        if (s == 0) n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), side);
+        if (s == 3 && early_peak) n += peak(side);
         CK(cudaEventRecord(ev_join, side));
         CK(cudaStreamWaitEvent(st, ev_join, 0));
       }
-      if (src.nsrc > 0) {
-        cgfd::SrcP q;
-        q.nsrc = src.nsrc; q.max_ext = src.max_ext; q.max_nt = src.max_nt;
-        q.force = src.force; q.moment = src.moment; q.stage = s;
-        q.ca = p.ca; q.cb = p.cb;
-        q.it_begin = d_it_begin; q.ext_num = d_ext_num; q.ext_idx = d_ext_idx;
-        q.ext_wv = d_ext_wv; q.ext_wt = d_ext_wt; q.stf = d_stf; q.src_shot = d_src_shot;
-        q.tmp_out = p.tmp_out; q.end = p.end; q.sf = sf; q.d_it = d_it; q.it_ahead = beside && s == 3;
-        q.wave16 = wave16; q.wsc = d_wsc; q.amax = d_amax;
-        n += timed(5, [&] { return cgfd::launch_source(q, st); });
-      }
+      if (src.nsrc > 0 && !src_in_tiles()) n += timed(5, [&] { return cgfd::launch_source(source_params(p, step), st); });
     }
     // drv_rk_curv_col.cu:519-527: after the last stage, before the level swap
     if (free_top && !early_peak) n += peak(st);
-    if (!fork) n += cgfd::launch_advance(d_it, st);
+    if (!fork) n += cgfd::launch_advance(d_it + (step & 1), d_it + (~step & 1), st);
     return n;
   }
 
@@ -917,7 +896,7 @@ void problem_bytes(const cgfd_problem_desc *d, int nshot, const cgfd_source_desc
   cgfd::recv_setup(d, rec);
   if (rec.n > 0)
     r += (size_t)rec.n * 8 * (sizeof(long long) + sizeof(float)) + (size_t)rec.n * 9 * d->nt_total * nshot * sizeof(float);
-  r += 2 * sizeof(int);
+  r += 3 * sizeof(int);
   if (d->free_top) r += (size_t)(15 * sizeof(float) + 3 * F) * d->ni * d->nj * nshot;
   if (w16) r += (size_t)nshot * (18 * F + 2 * sizeof(unsigned int) + (size_t)d->nt_total * 2 * F);
   if (resident) *resident = r;
@@ -1220,7 +1199,23 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
     size_t ne = (size_t)s.nsrc * s.max_ext;
     std::vector<long long> idx(ne, p->off0);
     for (size_t e = 0; e < ne; e++) idx[e] = p->didx(s.ext_i[e], s.ext_j[e], s.ext_k[e]);
-    for (size_t e = 0; e < ne; e++) p->src_top |= s.ext_k[e] == p->nk - 1;
+    // (more sources than this would be looked through by every tile that holds one)
+    constexpr int kTileSources = 64;
+    p->src_bulk = s.nsrc <= kTileSources;
+    for (int is = 0; is < s.nsrc; is++) {
+      cgfd_problem::Box b = {{INT_MAX, INT_MAX, INT_MAX}, {-1, -1, -1}};
+      for (int e = 0; e < s.ext_num[is]; e++) {
+        const size_t q = (size_t)is * s.max_ext + e;
+        const int at[3] = {s.ext_i[q], s.ext_j[q], s.ext_k[q]};
+        for (int a = 0; a < 3; a++) {
+          b.lo[a] = std::min(b.lo[a], at[a]);
+          b.hi[a] = std::max(b.hi[a], at[a]);
+        }
+      }
+      p->src_box.push_back(b);
+      p->src_top |= b.hi[2] == p->nk - 1;
+      p->src_bulk &= b.hi[2] < p->nbulk;
+    }
     p->d_it_begin = dmalloc<int>(s.nsrc, B, p->stream);
     p->d_ext_num = dmalloc<int>(s.nsrc, B, p->stream);
     p->d_ext_idx = dmalloc<long long>(ne, B, p->stream);
@@ -1285,9 +1280,9 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
     CK(cudaMemset(p->d_pg, 0, sizeof(float) * 15 * nij));
     CK(cudaMemset(p->d_dis, 0, E * 3 * nij));
   }
-  p->d_it = dmalloc<int>(1, B, p->stream);
+  p->d_it = dmalloc<int>(2, B, p->stream);
   p->d_flag = dmalloc<int>(1, B, p->stream);
-  CK(cudaMemset(p->d_it, 0, sizeof(int)));
+  CK(cudaMemset(p->d_it, 0, 2 * sizeof(int)));
   CK(cudaMemset(p->d_flag, 0, sizeof(int)));
   if (p->wave16) {
     p->d_wsc = dmalloc<float>(18 * (size_t)nshot, B, p->stream);
@@ -1480,10 +1475,21 @@ void make_tiles(cgfd_problem *p) {
       for (int g0 = 0; g0 < p->nshot; g0 += group)
         for (const int4 &e : list)
           for (int sh = g0; sh < std::min(p->nshot, g0 + group); sh++)
-            ex.push_back(make_int4(e.x + (sh << 16), e.y, e.z, e.w));
+            ex.push_back(make_int4(e.x + (sh << cgfd::kTileShotShift), e.y, e.z, e.w));
       list.swap(ex);
       npml *= p->nshot;
     }
+    if (p->med != cgfd::MED_AC && p->src_bulk)
+      for (int4 &e : list) {
+        const int lo[3] = {(e.x & cgfd::kTileBxMask) * cgfd::TX, e.y * ty, e.z};
+        const int hi[3] = {lo[0] + cgfd::TX - 1, lo[1] + ty - 1, e.w - 1};
+        for (int is = 0; is < p->src.nsrc; is++) {
+          const cgfd_problem::Box &b = p->src_box[is];
+          bool in = p->src_shot[is] == (e.x >> cgfd::kTileShotShift & cgfd::kTileShotMask);
+          for (int a = 0; a < 3; a++) in = in && b.lo[a] <= hi[a] && b.hi[a] >= lo[a];
+          if (in) e.x |= cgfd::kTileSource;
+        }
+      }
     int4 *&dt = dn ? p->d_tiles_dn : p->d_tiles;
     cgfd::BulkTiles &tl = dn ? p->tiles_dn : p->tiles;
     dfree(dt, p->stream);
@@ -1517,7 +1523,7 @@ void reset_state(cgfd_problem *p) {
   }
   if (p->d_amax) CK(cudaMemsetAsync(p->d_amax, 0, sizeof(unsigned int) * 2 * p->nshot, p->stream));
   p->it = 0;
-  CK(cudaMemsetAsync(p->d_it, 0, sizeof(int), p->stream));
+  CK(cudaMemsetAsync(p->d_it, 0, 2 * sizeof(int), p->stream));
   CK(cudaMemsetAsync(p->d_flag, 0, sizeof(int), p->stream));
   CK(cudaStreamSynchronize(p->stream));
   p->collect_timing();
@@ -1652,7 +1658,7 @@ int cgfd_set_step(cgfd_problem *p, int it) {
         if (p->graph_ok[s]) { cudaGraphExecDestroy(p->graph[s]); p->graph_ok[s] = false; }
     }
     p->it = it;
-    CK(cudaMemcpyAsync(p->d_it, &p->it, sizeof(int), cudaMemcpyHostToDevice, p->stream));
+    CK(cudaMemcpyAsync(p->d_it + (p->it & 1), &p->it, sizeof(int), cudaMemcpyHostToDevice, p->stream));
     refresh_wave_max(p);
     CK(cudaStreamSynchronize(p->stream));
   });

@@ -21,6 +21,7 @@
 
 #include "cgfd_dev.cuh"
 #include "cgfd_launch.h"
+#include "cgfd_source.cuh"
 #include "cgfd_tma.cuh"
 #include "cgfd_visco.cuh"
 
@@ -91,7 +92,8 @@ struct CoefTile {
 // is compiled out.
 // VIS: the visco-elastic form with that many mechanisms (0: elastic; vp is then unused).
 template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP, bool PML, int VIS = 0>
-__device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const TmaP &tm, const int4 tl, const VisP *vp = nullptr) {
+__device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const TmaP &tm, const int4 tl,
+                                          const SrcPT<real_of<TC>> &sp, const VisP *vp = nullptr) {
   using R = real_of<TC>;
   using TW = typename WavePolicy<WP, R>::TW;
   using TT = typename WavePolicy<WP, R>::TT;
@@ -105,7 +107,7 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem + S::OFF_BAR);  // NW wave, then 2 cpe
 
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int bx = tl.x & kTileBxMask, by = tl.y, shot = tl.x >> 16;
+  const int bx = tl.x & kTileBxMask, by = tl.y, shot = tl.x >> kTileShotShift & kTileShotMask;
   const int i = bx * TX + tx, j = by * TYT + ty;
   const int kb = tl.z, ke = tl.w;
   if (kb >= ke) return;
@@ -136,6 +138,14 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
     if (tid < 18) s_wsc[tid] = p.wsc[shot * 18 + tid];  // this shot's scale
   }
   __syncthreads();
+  // the shot's two scales (velocity, stress), held in registers: one shared-memory load per field and
+  // axis otherwise
+  [[maybe_unused]] float scale_v = 1.f, scale_s = 1.f;
+  if constexpr (WP == 2) {
+    scale_v = s_wsc[0];
+    scale_s = s_wsc[3];
+  }
+  auto scale = [&](int f) { return R(f < 3 ? scale_v : scale_s); };
 
   auto issue_wave = [&](int m) {
     const int kk = k0 + m * SD;
@@ -218,7 +228,7 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
         for (int f = 0; f < 9; f++) {
           const TW *r = W + f * S::WY * S::WX + (ty + LY) * S::WX + tx + S::XO - LX;
           d[f] = drp5<DX>(to_f(r[0]), to_f(r[1]), to_f(r[2]), to_f(r[3]), to_f(r[4]));
-          if constexpr (WP == 2) d[f] *= R(s_wsc[f]);  // the operator is linear: scale once
+          if constexpr (WP == 2) d[f] *= scale(f);  // the operator is linear: scale once
         }
       };
       auto deriv_y = [&](R d[9]) {
@@ -226,7 +236,7 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
         for (int f = 0; f < 9; f++) {
           const TW *r = W + f * S::WY * S::WX + ty * S::WX + tx + S::XO;
           d[f] = drp5<DY>(to_f(r[0]), to_f(r[S::WX]), to_f(r[2 * S::WX]), to_f(r[3 * S::WX]), to_f(r[4 * S::WX]));
-          if constexpr (WP == 2) d[f] *= R(s_wsc[f]);
+          if constexpr (WP == 2) d[f] *= scale(f);
         }
       };
       auto deriv_z = [&](R d[9]) {  // queue, this plane and the one ahead, in increasing k
@@ -234,7 +244,7 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
         for (int f = 0; f < 9; f++) {
           const R c0 = to_f(W[f * S::WY * S::WX + wc]), c1 = to_f(Wn[f * S::WY * S::WX + wc]);
           d[f] = SD > 0 ? drp5<DZ>(q[f][0], q[f][1], q[f][2], c0, c1) : drp5<DZ>(c1, c0, q[f][2], q[f][1], q[f][0]);
-          if constexpr (WP == 2) d[f] *= R(s_wsc[f]);
+          if constexpr (WP == 2) d[f] *= scale(f);
         }
       };
       CellAcc<R> acc;
@@ -334,6 +344,11 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
     fence_proxy_async_smem();
     __syncthreads();
   }
+  // sources inside the tile, after its stores (the last barrier orders them before these additions; the
+  // RK combine is linear, so this equals adding to the right-hand side). A launch of its own after
+  // every stage took 3-4 us of the critical path (100x100x60: 259 -> 250 us per step)
+  if (tl.x & kTileSource)
+    tile_sources(p, sp, shot, bx * TX, bx * TX + TX, by * TYT, by * TYT + TYT, kb, ke, tid, TX * TYT);
   if (bad) atomicOr(p.err, kErrWaveNonfinite);  // blow-up sentinel (drv_rk_curv_col.cu:507-510)
   if constexpr (WP == 2) {
     if (stage == 3) {  // the next step's FP16 scale
@@ -357,15 +372,15 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
 template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP>
 __global__ void __launch_bounds__(TX *TYT, BulkSmem<MED, TYT, TC, typename WavePolicy<WP, real_of<TC>>::TW, MINB>::BOUND)
     k_stage_bulk_tma(const __grid_constant__ StagePT<real_of<TC>> p, const __grid_constant__ TmaP tm,
-                     const int4 *__restrict__ tiles) {
+                     const __grid_constant__ SrcPT<real_of<TC>> sp, const int4 *__restrict__ tiles) {
   const int4 tl = __ldg(tiles + blockIdx.x);
-  if (tl.x & kTilePml) bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, true>(p, tm, tl);
-  else bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, false>(p, tm, tl);
+  if (tl.x & kTilePml) bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, true>(p, tm, tl, sp);
+  else bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, false>(p, tm, tl, sp);
 }
 
 // -----------------------------------------------------------------------------------------
 template <int MED, int SH, typename TC, int WP>
-static int launch_tma_shape(const StageP &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st) {
+static int launch_tma_shape(const StageP &p, const TmaP &tm, const SrcP &sp, const BulkTiles &t, cudaStream_t st) {
   constexpr int TYT = TileShape<MED, SH>::TYT, MINB = TileShape<MED, SH>::MINB;
   using S = BulkSmem<MED, TYT, TC, typename WavePolicy<WP>::TW, MINB>;
   if (t.n <= 0) return 0;
@@ -376,7 +391,7 @@ static int launch_tma_shape(const StageP &p, const TmaP &tm, const BulkTiles &t,
 #define CASE(c)                                                                                              \
   case c:                                                                                                    \
     k_stage_bulk_tma<MED, (c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1, TYT, MINB, TC, WP>                          \
-        <<<grid, block, S::BYTES, st>>>(p, tm, t.list);                                                      \
+        <<<grid, block, S::BYTES, st>>>(p, tm, sp, t.list);                                                      \
     break;
     CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7)
 #undef CASE
@@ -399,8 +414,8 @@ static cudaError_t set_attr_shape() {
 }
 
 template <int MED, typename TC, int WP>
-static int launch_tc(int shape, const StageP &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st) {
-  return shape ? launch_tma_shape<MED, 1, TC, WP>(p, tm, t, st) : launch_tma_shape<MED, 0, TC, WP>(p, tm, t, st);
+static int launch_tc(int shape, const StageP &p, const TmaP &tm, const SrcP &sp, const BulkTiles &t, cudaStream_t st) {
+  return shape ? launch_tma_shape<MED, 1, TC, WP>(p, tm, sp, t, st) : launch_tma_shape<MED, 0, TC, WP>(p, tm, sp, t, st);
 }
 
 template <int MED, typename TC, int WP>
@@ -410,16 +425,16 @@ static cudaError_t prepare_tc(int shape) {
 
 // One medium: every coefficient storage type and wave policy, both tile shapes.
 template <int MED>
-int launch_bulk_tma_med(int coef_type, int wave16, int shape, const StageP &p, const TmaP &tm, const BulkTiles &t,
-                        cudaStream_t st) {
+int launch_bulk_tma_med(int coef_type, int wave16, int shape, const StageP &p, const TmaP &tm, const SrcP &sp,
+                        const BulkTiles &t, cudaStream_t st) {
   if (wave16) {  // 16-bit fixed-point coefficients with FP16 stage levels
-    if (p.stage == 0) return launch_tc<MED, uint16_t, 1>(shape, p, tm, t, st);
-    return launch_tc<MED, uint16_t, 2>(shape, p, tm, t, st);
+    if (p.stage == 0) return launch_tc<MED, uint16_t, 1>(shape, p, tm, sp, t, st);
+    return launch_tc<MED, uint16_t, 2>(shape, p, tm, sp, t, st);
   }
-  if (coef_type == COEF_U16) return launch_tc<MED, uint16_t, 0>(shape, p, tm, t, st);
-  if (coef_type == COEF_F16) return launch_tc<MED, __half, 0>(shape, p, tm, t, st);
-  if (coef_type == COEF_BF16) return launch_tc<MED, __nv_bfloat16, 0>(shape, p, tm, t, st);
-  return launch_tc<MED, float, 0>(shape, p, tm, t, st);
+  if (coef_type == COEF_U16) return launch_tc<MED, uint16_t, 0>(shape, p, tm, sp, t, st);
+  if (coef_type == COEF_F16) return launch_tc<MED, __half, 0>(shape, p, tm, sp, t, st);
+  if (coef_type == COEF_BF16) return launch_tc<MED, __nv_bfloat16, 0>(shape, p, tm, sp, t, st);
+  return launch_tc<MED, float, 0>(shape, p, tm, sp, t, st);
 }
 
 template <int MED>

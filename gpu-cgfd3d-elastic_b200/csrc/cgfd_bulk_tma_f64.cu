@@ -11,7 +11,8 @@ template <> struct TileShape64<MED_ISO> { static constexpr int TYT = 4, MINB = 2
 template <> struct TileShape64<MED_VTI> { static constexpr int TYT = 8, MINB = 1; };
 
 template <int MED>
-static cudaError_t each_dir(int code, const StagePT<double> *p, const TmaP *tm, const BulkTiles *t, cudaStream_t st) {
+static cudaError_t each_dir(int code, const StagePT<double> *p, const TmaP *tm, const SrcPT<double> *sp, const BulkTiles *t,
+                            cudaStream_t st) {
   constexpr int TYT = TileShape64<MED>::TYT, MINB = TileShape64<MED>::MINB;
   using S = BulkSmem<MED, TYT, double, double, MINB>;
   static_assert(S::BYTES <= 227 * 1024, "one block must fit an SM's shared memory");
@@ -24,7 +25,7 @@ static cudaError_t each_dir(int code, const StagePT<double> *p, const TmaP *tm, 
           cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES);                                              \
   } else if (code == c) {                                                                                      \
     k_stage_bulk_tma<MED, (c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1, TYT, MINB, double, 0>                         \
-        <<<t->n, dim3(TX, TYT), S::BYTES, st>>>(*p, *tm, t->list);                                             \
+        <<<t->n, dim3(TX, TYT), S::BYTES, st>>>(*p, *tm, *sp, t->list);                                             \
   }
   CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7)
 #undef CASE
@@ -36,15 +37,16 @@ int tma64_tile_y(int med) { return med == MED_ISO ? TileShape64<MED_ISO>::TYT : 
 int tma64_resident(int med) { return med == MED_ISO ? TileShape64<MED_ISO>::MINB : TileShape64<MED_VTI>::MINB; }
 
 cudaError_t tma64_prepare(int med) {
-  return med == MED_ISO ? each_dir<MED_ISO>(0, nullptr, nullptr, nullptr, nullptr)
-                        : each_dir<MED_VTI>(0, nullptr, nullptr, nullptr, nullptr);
+  return med == MED_ISO ? each_dir<MED_ISO>(0, nullptr, nullptr, nullptr, nullptr, nullptr)
+                        : each_dir<MED_VTI>(0, nullptr, nullptr, nullptr, nullptr, nullptr);
 }
 
-int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st) {
+int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, const SrcPT<double> &sp,
+                            const BulkTiles &t, cudaStream_t st) {
   if (t.n <= 0) return 0;
   const int code = p.dir[0] | (p.dir[1] << 1) | (p.dir[2] << 2);
-  if (med == MED_ISO) each_dir<MED_ISO>(code, &p, &tm, &t, st);
-  else each_dir<MED_VTI>(code, &p, &tm, &t, st);
+  if (med == MED_ISO) each_dir<MED_ISO>(code, &p, &tm, &sp, &t, st);
+  else each_dir<MED_VTI>(code, &p, &tm, &sp, &t, st);
   return 1;
 }
 

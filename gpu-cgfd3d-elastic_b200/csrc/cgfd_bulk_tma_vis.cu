@@ -13,16 +13,16 @@ constexpr int kVisTY = 4, kVisBlocks = 4;
 template <int DX, int DY, int DZ, int NM>
 __global__ void __launch_bounds__(TX *kVisTY, kVisBlocks)
     k_stage_bulk_vis(const __grid_constant__ StageP p, const __grid_constant__ TmaP tm,
-                     const __grid_constant__ VisP v, const int4 *__restrict__ tiles) {
+                     const __grid_constant__ VisP v, const __grid_constant__ SrcP sp, const int4 *__restrict__ tiles) {
   const int4 tl = __ldg(tiles + blockIdx.x);
-  if (tl.x & kTilePml) bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, true, NM>(p, tm, tl, &v);
-  else bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, false, NM>(p, tm, tl, &v);
+  if (tl.x & kTilePml) bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, true, NM>(p, tm, tl, sp, &v);
+  else bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, false, NM>(p, tm, tl, sp, &v);
 }
 
 using VisSmem = BulkSmem<MED_ISO, kVisTY, float, float, kVisBlocks>;
 
 template <int NM>
-static cudaError_t for_each_dir(int code, const StageP *p, const TmaP *tm, const VisP *v, const BulkTiles *t,
+static cudaError_t for_each_dir(int code, const StageP *p, const TmaP *tm, const VisP *v, const SrcP *sp, const BulkTiles *t,
                                 cudaStream_t st) {
   cudaError_t e = cudaSuccess;
 #define CASE(c)                                                                                                  \
@@ -32,7 +32,7 @@ static cudaError_t for_each_dir(int code, const StageP *p, const TmaP *tm, const
                                cudaFuncAttributeMaxDynamicSharedMemorySize, VisSmem::BYTES);                     \
   } else if (code == c) {                                                                                        \
     k_stage_bulk_vis<(c)&1, ((c) >> 1) & 1, ((c) >> 2) & 1, NM>                                                  \
-        <<<t->n, dim3(TX, kVisTY), VisSmem::BYTES, st>>>(*p, *tm, *v, t->list);                                  \
+        <<<t->n, dim3(TX, kVisTY), VisSmem::BYTES, st>>>(*p, *tm, *v, *sp, t->list);                                  \
   }
   CASE(0) CASE(1) CASE(2) CASE(3) CASE(4) CASE(5) CASE(6) CASE(7)
 #undef CASE
@@ -42,22 +42,23 @@ static cudaError_t for_each_dir(int code, const StageP *p, const TmaP *tm, const
 int vis_bulk_max_mechanisms() { return 4; }
 int vis_bulk_resident() { return kVisBlocks; }
 
-static cudaError_t dispatch(int nmax, const StageP *p, const TmaP *tm, const VisP *v, const BulkTiles *t,
+static cudaError_t dispatch(int nmax, const StageP *p, const TmaP *tm, const VisP *v, const SrcP *sp, const BulkTiles *t,
                             cudaStream_t st) {
   const int code = p ? p->dir[0] | (p->dir[1] << 1) | (p->dir[2] << 2) : 0;
   switch (nmax) {
-    case 1: return for_each_dir<1>(code, p, tm, v, t, st);
-    case 2: return for_each_dir<2>(code, p, tm, v, t, st);
-    case 3: return for_each_dir<3>(code, p, tm, v, t, st);
-    default: return for_each_dir<4>(code, p, tm, v, t, st);
+    case 1: return for_each_dir<1>(code, p, tm, v, sp, t, st);
+    case 2: return for_each_dir<2>(code, p, tm, v, sp, t, st);
+    case 3: return for_each_dir<3>(code, p, tm, v, sp, t, st);
+    default: return for_each_dir<4>(code, p, tm, v, sp, t, st);
   }
 }
 
-cudaError_t tma_prepare_vis(int nmax) { return dispatch(nmax, nullptr, nullptr, nullptr, nullptr, nullptr); }
+cudaError_t tma_prepare_vis(int nmax) { return dispatch(nmax, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr); }
 
-int launch_stage_bulk_vis(const StageP &p, const TmaP &tm, const VisP &v, const BulkTiles &t, cudaStream_t st) {
+int launch_stage_bulk_vis(const StageP &p, const TmaP &tm, const VisP &v, const SrcP &sp, const BulkTiles &t,
+                          cudaStream_t st) {
   if (t.n <= 0) return 0;
-  dispatch(v.nmax, &p, &tm, &v, &t, st);
+  dispatch(v.nmax, &p, &tm, &v, &sp, &t, st);
   return 1;
 }
 

@@ -18,6 +18,7 @@
 
 #include "cgfd_dev.cuh"
 #include "cgfd_launch.h"
+#include "cgfd_source.cuh"
 #include "cgfd_tma.cuh"
 
 namespace cgfd {
@@ -462,38 +463,16 @@ __global__ void __launch_bounds__(32 * NSURF, 4) k_stage_surface(const __grid_co
 // One thread per (component, smoothing point): the kernel is a chain of dependent loads (step ->
 // time function -> weight) ended by one or two reductions, so its time is that chain's latency.
 // One thread per point with the 9 components in turn took 7.4 us per launch (343 points, one
-// source), four launches a step on the critical path of every grid; this form takes 3 us. The
-// reductions return no value except where the FP16 scale collector needs it.
+// source), four launches a step on the critical path of every grid; this form takes 3 us.
+// Sources below the surface slab are injected by the bulk stage's tiles instead where those run.
 template <typename R>
 __global__ void k_source(const __grid_constant__ SrcPT<R> s) {
   const int is = blockIdx.y, c = blockIdx.z;
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
   if (is >= s.nsrc || (c < 3 ? !s.force : !s.moment)) return;
-  const int it = *s.d_it - s.it_ahead;
-  const int ib = s.it_begin[is], ne = s.ext_num[is], shot = s.src_shot[is];
-  if (e >= ne || it < ib || it > ib + s.max_nt - 1) return;
-  const long long q = (long long)is * s.max_ext + e;
-  const long long id = s.ext_idx[q] + ((long long)shot * 9 + c) * s.sf;
-  const R w = (c < 3 ? s.ext_wv : s.ext_wt)[q];
-  const R v = s.stf[(((long long)is * s.max_nt + (it - ib)) * 4 + s.stage) * 9 + c];
-  const R h = c < 3 ? v * w : -v * w;
-  if (s.stage < 3) {
-    if constexpr (std::is_same<R, float>::value) {
-      if (s.wave16)
-        atomicAdd(reinterpret_cast<__half *>(s.tmp_out) + id, __float2half_rn(s.ca * h * s.wsc[18 * shot + 9 + c]));
-      else atomicAdd(s.tmp_out + id, s.ca * h);
-    } else {
-      atomicAdd(s.tmp_out + id, s.ca * h);
-    }
-  }
-  if constexpr (std::is_same<R, float>::value) {
-    if (s.wave16 && s.stage == 3) {
-      const R old = atomicAdd(s.end + id, s.cb * h);
-      atomic_max_abs(&s.amax[2 * shot + wgroup(c)], old + s.cb * h);
-      return;
-    }
-  }
-  atomicAdd(s.end + id, s.cb * h);
+  const int it = *s.d_it;
+  if (!source_active(s, is, it) || e >= s.ext_num[is]) return;
+  source_add(s, is, e, c, it, s.src_shot[is]);
 }
 
 template <typename R>
@@ -645,8 +624,9 @@ int launch_slices(const SliceP<R> &q, cudaStream_t st) {
 template int launch_slices<float>(const SliceP<float> &, cudaStream_t);
 template int launch_slices<double>(const SliceP<double> &, cudaStream_t);
 
-__global__ void k_advance(int *d_it) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *d_it += 1;
+// the next step's counter from this step's (steps of either parity read their own)
+__global__ void k_advance(const int *now, int *next) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) *next = *now + 1;
 }
 
 // Repack one field from the reference host layout (3 ghosts, nx = ni+6) into the device
@@ -984,8 +964,8 @@ int launch_recv(const RecvPT<R> &r, cudaStream_t st) {
 template int launch_recv<float>(const RecvPT<float> &, cudaStream_t);
 template int launch_recv<double>(const RecvPT<double> &, cudaStream_t);
 
-int launch_advance(int *d_it, cudaStream_t st) {
-  k_advance<<<1, 32, 0, st>>>(d_it);
+int launch_advance(const int *now, int *next, cudaStream_t st) {
+  k_advance<<<1, 32, 0, st>>>(now, next);
   return 1;
 }
 

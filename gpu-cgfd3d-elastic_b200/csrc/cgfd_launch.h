@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <climits>
+
 namespace cgfd {
 
 template <typename R> struct StagePT;
@@ -32,7 +34,6 @@ struct SrcPT {
   R *end;
   long long sf;
   const int *d_it;
-  int it_ahead;                // steps the counter is already ahead of the step being run (0 or 1)
   int wave16;                  // FP16 stage levels: tmp_out holds scaled __half
   const float *wsc;            // [nshot][18] scale / inverse scale of this step (wave16)
   unsigned int *amax;          // [nshot][2] max |w_end| per group, collected at stage 3 (wave16)
@@ -158,7 +159,9 @@ cudaError_t tma_prepare(int med, int coef_type, int wave16, int shape);
 // Tile list of the TMA bulk kernel (device array, one int4 per block in launch order:
 // bx + kTilePml if a CFS-PML face meets the tile + (shot << 16), by, first and end z plane).
 constexpr int kTilePml = 0x8000;     // bit 15 of x
-constexpr int kTileBxMask = 0x7fff;  // bits 0-14 of x: bx (bits 16-30: the shot)
+constexpr int kTileBxMask = 0x7fff;  // bits 0-14 of x: bx
+constexpr int kTileShotShift = 16, kTileShotMask = 0x7fff;  // bits 16-30: the shot
+constexpr int kTileSource = INT_MIN;  // bit 31: smoothing points of the shot's sources lie in the tile
 struct BulkTiles {
   const int4 *list = nullptr;
   int n = 0, npml = 0;  // entries, of which PML tiles
@@ -167,14 +170,16 @@ struct BulkTiles {
 int ac_tma_resident();
 cudaError_t ac_tma_prepare();
 int launch_stage_ac_tma(const StageP &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st);
+// sp: the sources that the tiles flagged kTileSource inject (nsrc 0: none)
 int launch_stage_bulk_tma(int med, int coef_type, int wave16, int shape, const StageP &p, const TmaP &tm,
-                          const BulkTiles &t, cudaStream_t st);
+                          const SrcP &sp, const BulkTiles &t, cudaStream_t st);
 // The FP64 build's TMA bulk kernel (iso and VTI media)
 bool tma64_supported(int med);
 int tma64_tile_y(int med);
 int tma64_resident(int med);
 cudaError_t tma64_prepare(int med);
-int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, const BulkTiles &t, cudaStream_t st);
+int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, const SrcPT<double> &sp,
+                            const BulkTiles &t, cudaStream_t st);
 // The visco-elastic form of the bulk kernel: the iso stage with the attenuation of the point and the
 // RK combine of the memory variables (v) between the right-hand side and the combine (32x4 tiles), for
 // up to vis_bulk_max_mechanisms() mechanisms (media with more run the direct-load kernel and the
@@ -182,7 +187,8 @@ int launch_stage_bulk_tma64(int med, const StagePT<double> &p, const TmaP &tm, c
 int vis_bulk_max_mechanisms();
 int vis_bulk_resident();  // blocks per SM
 cudaError_t tma_prepare_vis(int nmax);
-int launch_stage_bulk_vis(const StageP &p, const TmaP &tm, const VisP &v, const BulkTiles &t, cudaStream_t st);
+int launch_stage_bulk_vis(const StageP &p, const TmaP &tm, const VisP &v, const SrcP &sp, const BulkTiles &t,
+                          cudaStream_t st);
 // FP16 stage levels: per-step scale from the last step's max |w| and the step's source bound
 int launch_wave_scale(unsigned int *amax, const float *srcb, const int *d_it, int nt_total, int nshot, float *wsc,
                       cudaStream_t st);
@@ -203,7 +209,7 @@ template <typename R>
 int launch_source(const SrcPT<R> &s, cudaStream_t st);
 template <typename R>
 int launch_recv(const RecvPT<R> &r, cudaStream_t st);
-int launch_advance(int *d_it, cudaStream_t st);
+int launch_advance(const int *now, int *next, cudaStream_t st);
 // reference layout (float, 3 ghosts) -> device layout of real type R, and back
 template <typename R>
 void launch_repack_in(const float *src, R *dst, int ni, int nj, int nk, long long sx, long long sz,

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from cgfd_b200 import Simulation, media_layer_gpu, CGFD_MEDIA_ARI, CGFD_MEDIA_HAR, CGFD_PREC_FP64
+from cgfd_b200.abi import Sources
 from cgfd_b200.formats import LayerModel
 from helpers import small_problem, random_wavefield
 
@@ -132,3 +133,29 @@ def test_acoustic_tiles_equal_direct(grid, free_top, nshot):
     shots = [p.src] * nshot if nshot > 1 else None
     for a, b in zip(_two_steps(p, shots), _two_steps(p, shots, variant=0)):
         _close(a, b, 2e-5)  # components 4-8 stay 0 in both
+
+
+# inside a tile; across tile corners in x, y and z chunks; clipped by the grid's edge; reaching into the
+# surface slab's planes (then the source kernel runs); two that overlap
+@pytest.mark.parametrize("at", [[(40, 17, 9)], [(31, 8, 12)], [(0, 1, 2)], [(40, 17, 26)], [(33, 18, 11), (35, 20, 12)]])
+@pytest.mark.parametrize("medium,precision,tol", [("iso", 0, 2e-5), ("vis", 0, 2e-5), ("iso", CGFD_PREC_FP64, 1.2e-7)])
+@pytest.mark.parametrize("cmp_type", [1, 2])
+def test_sources_in_tiles_equal_source_kernel(at, medium, precision, tol, cmp_type):
+    n, steps = len(at), 5
+    p = small_problem(medium, 70, 41, 30, nsteps=steps, npml=3, nsrc=0)
+    p.precision = precision
+    rng = np.random.default_rng(2)
+    cmp = rng.uniform(-1, 1, (n, 9)).astype(np.float32) * np.array([1e12] * 3 + [1e16] * 6, np.float32)
+    coefs = np.zeros((n, 10), np.float32)
+    coefs[:, 0], coefs[:, 1] = 3.0, 0.02
+    p.src = Sources(loc=np.array(at, np.float32), t_start=np.zeros(n, np.float32), wavelet=np.zeros(n, np.int32),
+                    wavelet_coefs=coefs, cmp=cmp, stf_length=3 * p.dt, cmp_type=cmp_type)
+    out = []
+    for variant in (None, 0):
+        sim = Simulation(p)
+        if variant is not None:
+            sim.set_bulk_variant(variant)
+        sim.run(steps)  # the time function ends before the run does
+        out.append(sim.wavefield())
+    assert np.abs(out[1]).max() > 0
+    _close(out[0], out[1], tol)
