@@ -1425,10 +1425,10 @@ int default_chunk(const cgfd_problem *p) {
   return best;
 }
 
-// Tile lists of the TMA bulk kernel: 32 x TY columns, split along z into chunks of about
-// nzc planes that never straddle a z-face boundary of the CFS-PML (so planes above the
-// bottom absorbing layer run as tiles without face code); a tile that any PML face box meets
-// carries the kTilePml flag. Entries (bx [+ kTilePml] [+ shot << 16], by, first plane, end plane).
+// Tile lists of the TMA stage kernels: 32 x TY columns, split along z into chunks of about
+// nzc planes that never straddle a z-face boundary of the CFS-PML (so a column's faces are the same at
+// every plane of a tile). Entries (bx + flags + shot << 16, by, first plane, end plane): kTilePml on
+// tiles that a PML face box meets, kTileSource on those that hold sources.
 // Order: strips of tile rows, each strip z layer by z layer, x fastest. A strip's layer holds
 // about as many blocks as the GPU keeps resident, so that a tile's x-y neighbours run beside it
 // at the same planes (their halo lines are read from DRAM once), and the tile's next chunk

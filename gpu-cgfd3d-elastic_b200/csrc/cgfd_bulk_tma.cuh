@@ -1,5 +1,10 @@
 // cgfd_bulk_tma.cuh -- TMA-pipelined bulk RK-stage kernel for sm_100a (template; instantiated
-// per medium by cgfd_bulk_tma_{iso,vti,aniso}.cu, dispatched by cgfd_bulk_tma.cu).
+// per medium by cgfd_bulk_tma_{iso,vti,aniso}.cu, dispatched by cgfd_bulk_tma.cu; the visco-elastic
+// form by cgfd_bulk_tma_vis.cu, the FP64 build by cgfd_bulk_tma_f64.cu).
+//
+// What bounds it: DRAM traffic on large grids (480x480x240: 2.27 ms per stage for 12.5 GB, 0.85 of the
+// copy rate), and on grids with a large share of PML cells the instructions and memory round trips of
+// a plane at 16 warps per SM (5 shots of 141x118x77: 0.62 of the copy rate, IPC 1.5-2.0).
 //
 // Each thread block owns a 32 x TYT column tile and marches along z through its chunk of
 // planes. Thread 0 streams, two planes ahead of the computation and with mbarrier
@@ -88,10 +93,9 @@ struct CoefTile {
   __device__ __forceinline__ real_of<TC> operator()(int f) const { return coef_decode<TC>(c[f * STRIDE], p, f); }
 };
 
-// One tile (a block) of the stage; PML false: the tile meets no CFS-PML face and the face code
-// is compiled out.
+// One tile (a block) of the stage.
 // VIS: the visco-elastic form with that many mechanisms (0: elastic; vp is then unused).
-template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP, bool PML, int VIS = 0>
+template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP, int VIS = 0>
 __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const TmaP &tm, const int4 tl,
                                           const SrcPT<real_of<TC>> &sp, const VisP *vp = nullptr) {
   using R = real_of<TC>;
@@ -171,7 +175,7 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
   // PML faces that intersect this block (uniform), and those this thread's column lies in: z chunks
   // are cut at the z faces, so a column's faces are the same at every plane of the tile
   unsigned fmask = 0, tmask = 0;
-  for (int fi = 0; PML && fi < p.nface; fi++) {
+  for (int fi = 0; fi < p.nface; fi++) {
     const FacePT<R> &f = p.face[fi];
     const bool xo = f.lo[0] <= bx * TX + TX - 1 && f.hi[0] >= bx * TX;
     const bool yo = f.lo[1] <= by * TYT + TYT - 1 && f.hi[1] >= by * TYT;
@@ -263,39 +267,37 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
       h[1] = slw * acc.mom[1];
       h[2] = slw * acc.mom[2];
       md.hooke(acc.G, h + 3);
-      if constexpr (PML) {
-        // CFS-PML corrections added to the full right-hand side face by face, in face order
-        // (x1 x2 y1 y2 z1), as the reference applies its face kernels after the inner one;
-        // the face axis' derivatives are recomputed here, when the accumulators above are
-        // dead, to keep the face code's registers free
-        for (unsigned left = fmask; left; left &= left - 1) {
-          const int fi = __ffs(left) - 1;
-          if (!(tmask >> fi & 1)) continue;
-          const FacePT<R> &fc = p.face[fi];
-          R d[9];
-          auto face = [&](const R mrow[3]) {
-            pml_face<MED, (S::ONE_ROUND && VIS <= 2)>(p, fc, i, j, k, md, slw, mrow, d, d + 3, nullptr, nullptr, h, shot);
-          };
-          if constexpr (sizeof(R) == 4) {
-            // one copy of the face code for the three axes: it frees 10-16 registers, which hold what
-            // the auxiliaries' RK combine reads (in double the selected row costs more than that)
-            R mrow[3];
-            if (fc.axis == 0) deriv_x(d);
-            else if (fc.axis == 1) deriv_y(d);
-            else deriv_z(d);
+      // CFS-PML corrections added to the full right-hand side face by face, in face order
+      // (x1 x2 y1 y2 z1), as the reference applies its face kernels after the inner one;
+      // the face axis' derivatives are recomputed here, when the accumulators above are
+      // dead, to keep the face code's registers free
+      for (unsigned left = fmask; left; left &= left - 1) {
+        const int fi = __ffs(left) - 1;
+        if (!(tmask >> fi & 1)) continue;
+        const FacePT<R> &fc = p.face[fi];
+        R d[9];
+        auto face = [&](const R mrow[3]) {
+          pml_face<MED, (S::ONE_ROUND && VIS <= 2)>(p, fc, i, j, k, md, slw, mrow, d, d + 3, nullptr, nullptr, h, shot);
+        };
+        if constexpr (sizeof(R) == 4) {
+          // one copy of the face code for the three axes: it frees 10-16 registers, which hold what
+          // the auxiliaries' RK combine reads (in double the selected row costs more than that)
+          R mrow[3];
+          if (fc.axis == 0) deriv_x(d);
+          else if (fc.axis == 1) deriv_y(d);
+          else deriv_z(d);
 #pragma unroll
-            for (int c = 0; c < 3; c++) mrow[c] = fc.axis == 0 ? mt[0][c] : fc.axis == 1 ? mt[1][c] : mt[2][c];
-            face(mrow);
-          } else if (fc.axis == 0) {
-            deriv_x(d);
-            face(mt[0]);
-          } else if (fc.axis == 1) {
-            deriv_y(d);
-            face(mt[1]);
-          } else {
-            deriv_z(d);
-            face(mt[2]);
-          }
+          for (int c = 0; c < 3; c++) mrow[c] = fc.axis == 0 ? mt[0][c] : fc.axis == 1 ? mt[1][c] : mt[2][c];
+          face(mrow);
+        } else if (fc.axis == 0) {
+          deriv_x(d);
+          face(mt[0]);
+        } else if (fc.axis == 1) {
+          deriv_y(d);
+          face(mt[1]);
+        } else {
+          deriv_z(d);
+          face(mt[2]);
         }
       }
       const long long id = didx(p, i, j, k);
@@ -365,17 +367,17 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
 }
 
 
-// The bulk stage: one block per tile-list entry, in list order. An entry is (bx + PML flag
-// (kTilePml) + (shot << 16), by, first plane, end plane); a PML tile runs the face code, the
-// others its compiled-out form. Both kinds in one launch keep a tile's x-y neighbours, PML or
-// not, resident beside it, so that the halo lines they share are read from DRAM once.
+// The bulk stage: one block per tile-list entry, in list order. An entry is (bx + flags + (shot << 16),
+// by, first plane, end plane). Every tile runs the same code, PML or not: a second body without the
+// face code for the tiles no face meets kept both out of the instruction cache (us per step, two bodies
+// against one: 8 mixed shots of 128x128x64 1984 / 1922, visco-elastic 160x160x80 1140 / 1103, 5 shots
+// of 141x118x77 1636 / 1620, 480x480x240 9588 / 9576).
 template <int MED, int DX, int DY, int DZ, int TYT, int MINB, typename TC, int WP>
 __global__ void __launch_bounds__(TX *TYT, BulkSmem<MED, TYT, TC, typename WavePolicy<WP, real_of<TC>>::TW, MINB>::BOUND)
     k_stage_bulk_tma(const __grid_constant__ StagePT<real_of<TC>> p, const __grid_constant__ TmaP tm,
                      const __grid_constant__ SrcPT<real_of<TC>> sp, const int4 *__restrict__ tiles) {
   const int4 tl = __ldg(tiles + blockIdx.x);
-  if (tl.x & kTilePml) bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, true>(p, tm, tl, sp);
-  else bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP, false>(p, tm, tl, sp);
+  bulk_tile<MED, DX, DY, DZ, TYT, MINB, TC, WP>(p, tm, tl, sp);
 }
 
 // -----------------------------------------------------------------------------------------

@@ -15,8 +15,7 @@ __global__ void __launch_bounds__(TX *kVisTY, kVisBlocks)
     k_stage_bulk_vis(const __grid_constant__ StageP p, const __grid_constant__ TmaP tm,
                      const __grid_constant__ VisP v, const __grid_constant__ SrcP sp, const int4 *__restrict__ tiles) {
   const int4 tl = __ldg(tiles + blockIdx.x);
-  if (tl.x & kTilePml) bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, true, NM>(p, tm, tl, sp, &v);
-  else bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, false, NM>(p, tm, tl, sp, &v);
+  bulk_tile<MED_ISO, DX, DY, DZ, kVisTY, kVisBlocks, float, 0, NM>(p, tm, tl, sp, &v);
 }
 
 using VisSmem = BulkSmem<MED_ISO, kVisTY, float, float, kVisBlocks>;

@@ -1,5 +1,5 @@
 // cgfd_bulk_tma_vti.cu -- the bulk RK-stage kernel's instantiations for the vti medium (every
-// operator direction, coefficient storage, wave policy, PML / interior variant and tile shape).
+// operator direction, coefficient storage, wave policy and tile shape).
 #include "cgfd_bulk_tma.cuh"
 
 namespace cgfd {

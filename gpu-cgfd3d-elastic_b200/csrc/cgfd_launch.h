@@ -156,9 +156,9 @@ int tma_blocks_per_sm(int med, int shape);  // resident blocks per SM the tile s
 // 128 registers per thread)
 int tma_resident(int med, int coef_type, int wave16, int shape);
 cudaError_t tma_prepare(int med, int coef_type, int wave16, int shape);
-// Tile list of the TMA bulk kernel (device array, one int4 per block in launch order:
-// bx + kTilePml if a CFS-PML face meets the tile + (shot << 16), by, first and end z plane).
-constexpr int kTilePml = 0x8000;     // bit 15 of x
+// Tile list of the TMA stage kernels (device array, one int4 per block in launch order:
+// bx + flags + (shot << 16), by, first and end z plane).
+constexpr int kTilePml = 0x8000;     // bit 15 of x: a CFS-PML face meets the tile (acoustic kernel)
 constexpr int kTileBxMask = 0x7fff;  // bits 0-14 of x: bx
 constexpr int kTileShotShift = 16, kTileShotMask = 0x7fff;  // bits 16-30: the shot
 constexpr int kTileSource = INT_MIN;  // bit 31: smoothing points of the shot's sources lie in the tile
