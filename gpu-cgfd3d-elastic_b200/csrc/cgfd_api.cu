@@ -657,7 +657,14 @@ struct cgfd_problem {
         if (!graph_ok[slot]) {
           cudaGraph_t g;
           CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-          graph_launches[slot] = enqueue_step(step);
+          try {
+            graph_launches[slot] = enqueue_step(step);
+          } catch (...) {  // leave no stream in capture behind
+            g = nullptr;
+            cudaStreamEndCapture(stream, &g);
+            if (g) cudaGraphDestroy(g);
+            throw;
+          }
           CK(cudaStreamEndCapture(stream, &g));
           CK(cudaGraphInstantiate(&graph[slot], g, 0));
           CK(cudaGraphDestroy(g));
@@ -1293,7 +1300,10 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
     p->d_srcb = dmalloc<float>(sb.size(), B, p->stream);
     CK(cudaMemcpy(p->d_srcb, sb.data(), sb.size() * sizeof(float), cudaMemcpyHostToDevice));
   }
-  CK(cudaDeviceSynchronize());
+  // this problem's work only (its stream, and the legacy stream of the copies and fills above): a
+  // device-wide wait is not allowed while another thread captures a step of its own problem
+  CK(cudaStreamSynchronize(cudaStreamLegacy));
+  CK(cudaStreamSynchronize(p->stream));
 }
 
 // TMA tensor maps of the four wavefield levels and of the coefficients for the current tile
