@@ -72,7 +72,7 @@ extern "C" {
 #define CGFD_PREC_FP64       5  /* FP64 build of the same kernels: wavefield, coefficients, PML
                                    auxiliaries and all arithmetic in double (the reference
                                    each precision mode's seismogram error is measured against;
-                                   direct-load bulk kernel, not a production mode)            */
+                                   not a production mode)                                     */
 
 /* status codes */
 #define CGFD_OK               0
@@ -383,7 +383,8 @@ int cgfd_get_shot_group(const cgfd_problem *p);
 int cgfd_autotune(cgfd_problem *p, int steps, int *chosen);
 
 /* Bulk stage kernel variant: 1 = TMA-pipelined (default), 0 = direct global loads. Acoustic
-   media: their stage kernel in the same two forms (FP32; the FP64 build runs direct loads). */
+   media: their stage kernel in the same two forms (FP32; the FP64 build runs direct loads). The FP64
+   build and visco-elastic media take 0 only (their own TMA kernels run until then). */
 int cgfd_set_bulk_variant(cgfd_problem *p, int tma);
 
 /* Per-kernel CUDA-event timing of subsequent steps (uses direct launches while on). */
