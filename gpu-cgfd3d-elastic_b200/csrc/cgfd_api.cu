@@ -1658,9 +1658,11 @@ int cgfd_set_step(cgfd_problem *p, int it) {
   return guarded([&] {
     CK(cudaSetDevice(p->device));
     CK(cudaStreamSynchronize(p->stream));
-    // the buffer roles follow the step parity: move w_pre / PML pre to the new parity
+    // the buffer roles follow the step parity: move w_pre, the PML pre level and the memory
+    // variables of visco-elastic media to the new parity
     if ((it & 1) != (p->it & 1)) {
       std::swap(p->wbuf[0], p->wbuf[1]);
+      std::swap(p->jbuf[0], p->jbuf[1]);
       std::swap(p->map_halo[0], p->map_halo[1]);
       std::swap(p->map_ctr[0], p->map_ctr[1]);
       p->aux_flip ^= 1;
