@@ -689,10 +689,19 @@ template <typename R>
 int launch_stage_bulk(int med, const StagePT<R> &p, int nzc, cudaStream_t st) {
   if (p.nbulk <= 0) return 0;
   dim3 grid((p.ni + TX - 1) / TX, (p.nj + TY - 1) / TY, (p.nbulk + nzc - 1) / nzc);
-  if (med == MED_ISO) launch_bulk_med<MED_ISO>(p, nzc, grid, st);
-  else if (med == MED_VTI) launch_bulk_med<MED_VTI>(p, nzc, grid, st);
-  else launch_bulk_med<MED_ANISO>(p, nzc, grid, st);
-  return 1;
+  for (int shot = 0; shot < p.nshot; shot++) {  // the kernel advances one shot (batches: 21-Cij media in FP64)
+    StagePT<R> q = p;
+    const long long w = (long long)shot * 9 * p.sf;
+    q.cur += w;
+    q.pre += w;
+    if (q.tmp_out) q.tmp_out += w;
+    q.end += w;
+    for (int f = 0; f < p.nface; f++) q.face[f].aux += shot * p.face[f].shot * kAuxBlock;
+    if (med == MED_ISO) launch_bulk_med<MED_ISO>(q, nzc, grid, st);
+    else if (med == MED_VTI) launch_bulk_med<MED_VTI>(q, nzc, grid, st);
+    else launch_bulk_med<MED_ANISO>(q, nzc, grid, st);
+  }
+  return p.nshot;
 }
 template int launch_stage_bulk<float>(int, const StagePT<float> &, int, cudaStream_t);
 template int launch_stage_bulk<double>(int, const StagePT<double> &, int, cudaStream_t);

@@ -131,7 +131,7 @@ int launch_slices(const SliceP<R> &q, cudaStream_t st);
 void launch_metric(const float *x, const float *y, const float *z, float *const out[10], int ni, int nj, int nk,
                    long long sx, long long sz, long long off0, cudaStream_t st);
 
-// Each launcher returns the number of kernels it launched (0 or 1).
+// Each launcher returns the number of kernels it launched (0 or 1; launch_stage_bulk: one per shot).
 template <typename R>
 int launch_stage_bulk(int med, const StagePT<R> &p, int nzc, cudaStream_t st);
 int launch_stage_surface(int med, int coef_type, int wave16, const StageP &p, cudaStream_t st);

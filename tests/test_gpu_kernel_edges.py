@@ -159,3 +159,22 @@ def test_sources_in_tiles_equal_source_kernel(at, medium, precision, tol, cmp_ty
         out.append(sim.wavefield())
     assert np.abs(out[1]).max() > 0
     _close(out[0], out[1], tol)
+
+
+@pytest.mark.parametrize("medium", ["iso", "aniso", "ac"])
+def test_fp64_batch_equals_its_shots_alone(medium):
+    p = small_problem(medium, 40, 37, 30, nsteps=8, npml=4, nsrc=1)
+    p.precision = CGFD_PREC_FP64
+    waves = [random_wavefield(p, seed=s) for s in (1, 2, 3)]
+    if medium == "ac":
+        for w in waves:
+            w[4:] = 0
+
+    def run(shots, state):
+        with Simulation(p, shots) as sim:
+            for s, w in enumerate(state):
+                sim.set_wavefield(w, s)
+            sim.run(4)
+            return [sim.wavefield(s) for s in range(sim.nshot)]
+    for got, w in zip(run([p.src] * 3, waves), waves):
+        np.testing.assert_array_equal(got, run(None, [w])[0])
