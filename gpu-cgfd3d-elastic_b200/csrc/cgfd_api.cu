@@ -724,6 +724,16 @@ int guarded(Fn fn) {
   }
 }
 
+// Host array -> device array that the problem's steps read. In the order of the problem's stream: a
+// copy on the legacy stream is not ordered with that stream (it is a non-blocking one), and a copy
+// from pageable memory may return before it has reached the device. Returns when it has (the host
+// array may go).
+void upload(cgfd_problem *p, void *dst, const void *src, size_t bytes) {
+  if (bytes == 0) return;
+  CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, p->stream));
+  CK(cudaStreamSynchronize(p->stream));
+}
+
 // One model field (reference layout) into its device array, through stage_buf. ps: the
 // device's pinned stager, its lock held by the caller (nullptr: plain pageable copy).
 // dst: the device field (float, or double in the FP64 build).
@@ -1506,7 +1516,7 @@ void make_tiles(cgfd_problem *p) {
     dt = nullptr;
     size_t acc = 0;
     dt = dmalloc<int4>(std::max<size_t>(list.size(), 1), acc, p->stream);
-    if (!list.empty()) CK(cudaMemcpy(dt, list.data(), list.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    upload(p, dt, list.data(), list.size() * sizeof(int4));
     tl.list = dt;
     tl.n = (int)list.size();
     tl.npml = npml;
@@ -1636,8 +1646,7 @@ int cgfd_check_wait_bound(cgfd_problem *p) {
   if (rc != CGFD_OK) return rc;
   rc = cgfd_synchronize(p);  // reports the timeout like a stage kernel's
   std::string msg = g_err;
-  int zero = 0;
-  if (cudaMemcpy(p->d_flag, &zero, sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemsetAsync(p->d_flag, 0, sizeof(int), p->stream) != cudaSuccess) {
     set_err("could not clear the device error word");
     return CGFD_ERR_CUDA;
   }
@@ -1904,9 +1913,9 @@ int cgfd_set_line_receivers(cgfd_problem *p, int npts, const int *ijk) {
       p->d_line_idx8 = dmalloc<long long>(idx.size(), p->bytes, p->stream);
       p->d_line_w8 = dmalloc<float>(w.size(), p->bytes, p->stream);
       p->d_line_seis = dmalloc<float>((size_t)npts * 9 * p->nt_total * p->nshot, p->bytes, p->stream);
-      CK(cudaMemcpy(p->d_line_idx8, idx.data(), idx.size() * sizeof(long long), cudaMemcpyHostToDevice));
-      CK(cudaMemcpy(p->d_line_w8, w.data(), w.size() * sizeof(float), cudaMemcpyHostToDevice));
-      CK(cudaMemset(p->d_line_seis, 0, sizeof(float) * npts * 9 * p->nt_total * p->nshot));
+      upload(p, p->d_line_idx8, idx.data(), idx.size() * sizeof(long long));
+      upload(p, p->d_line_w8, w.data(), w.size() * sizeof(float));
+      CK(cudaMemsetAsync(p->d_line_seis, 0, sizeof(float) * npts * 9 * p->nt_total * p->nshot, p->stream));
       p->nline = npts;
     }
     for (int s = 0; s < 8; s++)
@@ -1953,7 +1962,7 @@ int cgfd_set_slices(cgfd_problem *p, int nx, const int *ix, int ny, const int *i
       idx.insert(idx.end(), iy, iy + ny);
       idx.insert(idx.end(), iz, iz + nz);
       p->d_slice_idx = dmalloc<int>(idx.size(), p->bytes, p->stream);
-      CK(cudaMemcpy(p->d_slice_idx, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice));
+      upload(p, p->d_slice_idx, idx.data(), idx.size() * sizeof(int));
       p->d_slices = dmalloc<float>((size_t)ring_steps * p->nshot * per, p->bytes, p->stream);
       p->nslx = nx; p->nsly = ny; p->nslz = nz;
       p->slice_ring = ring_steps;
