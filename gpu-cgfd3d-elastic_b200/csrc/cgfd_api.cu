@@ -334,9 +334,11 @@ struct cgfd_problem {
     return p;
   }
 
-  // whether the bulk (acoustic: whole) stage runs from tile lists; tile height, and blocks per SM of
-  // the kernel that does (strip_blocks: those the strips of the tile order are sized for)
+  // whether the bulk (acoustic: whole) stage can run from tile lists, and whether it does; tile height,
+  // and blocks per SM of the kernel that does (strip_blocks: those the strips of the tile order are sized
+  // for)
   bool tiled() const { return med != cgfd::MED_AC || ac_tiled; }
+  bool runs_tiles() const { return use_tma || vis_tma || tma64 || ac_tma; }
   int tile_y() const {
     return med == cgfd::MED_AC ? cgfd::TY : tma64 ? cgfd::tma64_tile_y(med) : cgfd::tma_tile_y(med, shape);
   }
@@ -1414,7 +1416,7 @@ int default_chunk(const cgfd_problem *p) {
   if (p->nbulk < 1) return 1;
   int nsm = 148;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device));
-  const bool tiled = p->use_tma || p->vis_tma || p->tma64 || p->ac_tma;
+  const bool tiled = p->runs_tiles();
   const int ty = tiled ? p->tile_y() : cgfd::TY;
   const long long resident = (long long)nsm * p->resident_blocks();
   const long long columns = (long long)((p->ni + cgfd::TX - 1) / cgfd::TX) * ((p->nj + ty - 1) / ty) * p->nshot;
@@ -2063,7 +2065,7 @@ int cgfd_set_shot_group(cgfd_problem *p, int group) {
     CK(cudaSetDevice(p->device));
     CK(cudaStreamSynchronize(p->stream));
     p->shot_group = group;
-    if (p->use_tma) make_tiles(p);  // the strip height follows the group
+    make_tiles(p);  // the strip height follows the group
     for (int s = 0; s < 8; s++)
       if (p->graph_ok[s]) { cudaGraphExecDestroy(p->graph[s]); p->graph_ok[s] = false; }
   });
@@ -2149,7 +2151,7 @@ int cgfd_autotune(cgfd_problem *p, int steps, int *chosen) {
     p->nzc = best;
     make_tiles(p);
     // batches: the shot group at the chosen tiling (4, 8, 16 or every shot)
-    if (p->use_tma && p->nshot > 1) {
+    if (p->runs_tiles() && p->nshot > 1) {
       int best_g = std::max(1, std::min(p->shot_group, p->nshot));
       float best_gms = 1e30f;
       std::vector<int> gc;

@@ -72,3 +72,27 @@ def test_shot_groups_agree_and_autotune_picks_one():
     b.run()
     assert np.array_equal(b.seismograms(), ref[0])
     b.close()
+
+
+@pytest.mark.parametrize("medium,precision", [("ac", 0), ("iso", 5)])
+def test_shot_groups_of_acoustic_and_fp64_batches(medium, precision):
+    """These run from the same tile lists: a group takes effect at once and changes no result, and the
+    autotuner picks one."""
+    p = small_problem(medium, nsteps=20, nsrc=0)
+    p.precision = precision
+    shots = _shots(p, 5, 9)
+    ref = None
+    for g in (5, 1, 2):
+        with Simulation(p, shots=shots) as b:
+            b.set_shot_group(g)
+            b.run()
+            out = [b.seismograms()] + [b.wavefield(n) for n in range(5)]
+        ref = ref or out
+        for x, y in zip(out, ref):
+            assert np.array_equal(x, y)
+    with Simulation(p, shots=shots) as b:
+        b.set_shot_group(1)
+        b.autotune(2)
+        assert b.shot_group in (4, 5)
+        b.run()
+        assert np.array_equal(b.seismograms(), ref[0])
