@@ -759,6 +759,10 @@ int layer_iso_family(int device, int ni, int nj, int nk, const float *coord, int
       cleanup();
       set_last_error(x.what());
       return x.code;
+    } catch (const std::exception &x) {
+      cleanup();
+      set_last_error(x.what());
+      return CGFD_ERR_INVALID;
     }
   } else if ((e = cudaMemcpyAsync(medium, dout, bytes, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
     return fail(e, "cudaMemcpy");

@@ -29,7 +29,8 @@ namespace cgfd {
 // of the process (2 x 64 MiB of pinned host memory): allocating and freeing pinned memory per
 // problem would synchronise the device under the serving loop's concurrent problems. Users
 // hold its lock for a whole upload; each chunk is refilled only after the copy out of it
-// has completed (per-chunk events), so no device-wide synchronisation is involved.
+// has completed (per-chunk events), so no device-wide synchronisation is involved. Where the host has
+// no pinned memory to give, transfers take the plain pageable copy.
 class PinnedStager {
  public:
   static constexpr size_t kChunk = size_t(64) << 20;
@@ -44,7 +45,7 @@ class PinnedStager {
     static std::vector<PinnedStager *> all;
     std::lock_guard<std::mutex> lk(mu);
     if ((int)all.size() <= device) all.resize(device + 1, nullptr);
-    if (!all[device]) all[device] = new PinnedStager();  // device is current
+    if (!all[device]) all[device] = new PinnedStager();
     return *all[device];
   }
   std::mutex &mutex() { return mu_; }
@@ -65,6 +66,13 @@ class PinnedStager {
       CGFD_CK(cudaEventRecord(done_[c & 1], st));
     };
     if (nch == 0) return;
+    if (!ready()) {
+      for (int q = 0; q < parts; q++) {
+        produce(q);
+        CGFD_CK(cudaMemcpyAsync(static_cast<char *>(dst) + q * n, src, n, cudaMemcpyDeviceToHost, st));
+      }
+      return;
+    }
     issue(0);
     for (size_t c = 0; c < nch; c++) {
       if (c + 1 < nch) issue(c + 1);
@@ -85,6 +93,10 @@ class PinnedStager {
   }
 
   void copy(void *dst, const void *src, size_t n, cudaStream_t st) {
+    if (!ready()) {
+      CGFD_CK(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st));
+      return;
+    }
     for (size_t o = 0; o < n; o += kChunk) {
       const size_t m = std::min(kChunk, n - o);
       const int b = next_;
@@ -103,11 +115,17 @@ class PinnedStager {
   }
 
  private:
-  PinnedStager() {
+  PinnedStager() = default;
+  bool ready() {  // both chunks, allocated on first use (the device is current)
     for (int b = 0; b < 2; b++) {
-      CGFD_CK(cudaHostAlloc(reinterpret_cast<void **>(&buf_[b]), kChunk, cudaHostAllocPortable));
-      CGFD_CK(cudaEventCreateWithFlags(&done_[b], cudaEventDisableTiming));
+      if (!done_[b]) CGFD_CK(cudaEventCreateWithFlags(&done_[b], cudaEventDisableTiming));
+      if (!buf_[b] && cudaHostAlloc(reinterpret_cast<void **>(&buf_[b]), kChunk, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        buf_[b] = nullptr;
+        return false;
+      }
     }
+    return true;
   }
   static constexpr size_t kPiece = size_t(1) << 18;
   std::mutex mu_;
