@@ -87,3 +87,14 @@ def test_transfers_are_whole_with_and_without_pinned_memory(program, grants):
     pinned = _run(program, grants, "o:1:3", f"o:{3 * mib + 5}:9", f"i:{64 * mib}", f"o:{64 * mib + 1}:2", "i:0", "o:0:1",
                   f"i:{130 * mib + 7}", f"o:{128 * mib}:1", "i:12345")
     assert (pinned[-1] > 0) == (grants > 0)
+
+
+def test_short_transfers_take_little_pinned_memory(program):
+    """A third of a transfer's bytes, rounded up to a piece of 8 MiB for each of the two chunks, and twice
+    64 MiB at most; a later transfer takes what an earlier one had."""
+    mib = 1 << 20
+    first, second, third, last = _run(program, 100, f"o:{45 * mib}:1", f"o:{20 * mib}:9", f"i:{100 * mib}", f"o:{260 * mib}:2")
+    assert first <= 45 * mib / 3 + 2 * 8 * mib
+    assert second <= 180 * mib / 3 + 2 * 8 * mib
+    assert third == second
+    assert last == 128 * mib
