@@ -188,7 +188,8 @@ struct cgfd_problem {
 
   cgfd::SrcHost src;
   bool src_top = false;  // a source's smoothing points reach the top plane
-  bool src_bulk = false;  // at most kTileSources sources, no smoothing point in the surface slab
+  bool src_bulk = false;  // at most one source a shot and kTileSources in all, none reaching the surface slab
+  bool src_tiles = false;  // and none in a tile where faces of two axes meet (make_tiles)
   struct Box { int lo[3], hi[3]; };
   std::vector<Box> src_box;  // of each source's smoothing points
   std::vector<int> src_shot;
@@ -354,9 +355,16 @@ struct cgfd_problem {
     return cgfd::tma_resident(med, coef_type, wave16, shape);
   }
 
-  // Sources whose smoothing points all lie in the bulk planes, few enough for a tile to look through,
-  // are injected by the tiles of the TMA stage kernels (kTileSource); others by the source kernel.
-  bool src_in_tiles() const { return src_bulk && (use_tma || vis_tma || tma64); }
+  // Sources injected by the tiles of the TMA stage kernels that hold them (kTileSource), which saves the
+  // source kernel's launch after every stage; a block adds its sources one after the other when its tile
+  // is done, so only where that does not lengthen the stage: one source a shot, whose smoothing points
+  // lie in the bulk planes and in no tile where CFS-PML faces of two axes meet (those take longest). us
+  // per step, tile / source kernel: one source inside 64x64x64 107 / 113 (FP64 195 / 205, visco-elastic
+  // 194 / 201), 100x100x60 282 / 280 (mixed storage 263 / 278, 21-Cij 281 / 291), 200x200x100 937 / 949;
+  // in an edge or corner of 64x64x64 127 / 113, 100x100x60 322 / 280 (mixed 353 / 278); two sources in one
+  // region 64x64x64 117 / 113, 100x100x60 mixed 295 / 279; 64 there 1310 / 115 and 4377 / 371. Shots
+  // with one source each: 2 to 32 of 64x64x64 0-2% faster in tiles, 64 0.2% slower.
+  bool src_in_tiles() const { return src_tiles && (use_tma || vis_tma || tma64); }
 
   template <typename R>
   cgfd::SrcPT<R> source_params(const cgfd::StagePT<R> &p, int step) const {
@@ -1218,9 +1226,10 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
     size_t ne = (size_t)s.nsrc * s.max_ext;
     std::vector<long long> idx(ne, p->off0);
     for (size_t e = 0; e < ne; e++) idx[e] = p->didx(s.ext_i[e], s.ext_j[e], s.ext_k[e]);
-    // (more sources than this would be looked through by every tile that holds one)
-    constexpr int kTileSources = 64;
-    p->src_bulk = s.nsrc <= kTileSources;
+    constexpr int kTileSources = 32;
+    std::vector<int> of_shot(p->nshot, 0);
+    for (int sh : p->src_shot) of_shot[sh]++;
+    p->src_bulk = s.nsrc <= kTileSources && *std::max_element(of_shot.begin(), of_shot.end()) <= 1;
     for (int is = 0; is < s.nsrc; is++) {
       cgfd_problem::Box b = {{INT_MAX, INT_MAX, INT_MAX}, {-1, -1, -1}};
       for (int e = 0; e < s.ext_num[is]; e++) {
@@ -1468,6 +1477,27 @@ void make_tiles(cgfd_problem *p) {
   const int group = std::max(1, std::min(p->shot_group, p->nshot));
   const long long resident = (long long)nsm * p->strip_blocks();
   const int strip = (int)std::max<long long>(1, (resident + (long long)nbx * group - 1) / ((long long)nbx * group));
+  // axes (bits) of the CFS-PML faces that meet a tile
+  auto face_axes = [&](int bx, int by, const std::pair<int, int> &z) {
+    int axes = 0;
+    for (const auto &f : p->faces) {
+      const bool xo = f.h.lo[0] <= bx * cgfd::TX + cgfd::TX - 1 && f.h.hi[0] >= bx * cgfd::TX;
+      const bool yo = f.h.lo[1] <= by * ty + ty - 1 && f.h.hi[1] >= by * ty;
+      const bool zo = f.h.lo[2] <= z.second - 1 && f.h.hi[2] >= z.first;
+      if (xo && yo && zo) axes |= 1 << f.h.axis;
+    }
+    return axes;
+  };
+  p->src_tiles = p->src_bulk;
+  if (p->src_tiles)
+    for (const cgfd_problem::Box &b : p->src_box)
+      for (const auto &z : zr)
+        if (b.lo[2] < z.second && b.hi[2] >= z.first)
+          for (int by = b.lo[1] / ty; by <= b.hi[1] / ty; by++)
+            for (int bx = b.lo[0] / cgfd::TX; bx <= b.hi[0] / cgfd::TX; bx++) {
+              const int axes = face_axes(bx, by, z);
+              if (axes & (axes - 1)) p->src_tiles = false;
+            }
   for (int dn = 0; dn < 2; dn++) {
     std::vector<int4> list;
     int npml = 0;
@@ -1476,13 +1506,7 @@ void make_tiles(cgfd_problem *p) {
         const auto &z = zr[dn ? zr.size() - 1 - zi : zi];
         for (int by = s0; by < std::min(nby, s0 + strip); by++)
           for (int bx = 0; bx < nbx; bx++) {
-            bool touch = false;
-            for (const auto &f : p->faces) {
-              const bool xo = f.h.lo[0] <= bx * cgfd::TX + cgfd::TX - 1 && f.h.hi[0] >= bx * cgfd::TX;
-              const bool yo = f.h.lo[1] <= by * ty + ty - 1 && f.h.hi[1] >= by * ty;
-              const bool zo = f.h.lo[2] <= z.second - 1 && f.h.hi[2] >= z.first;
-              touch |= xo && yo && zo;
-            }
+            const bool touch = face_axes(bx, by, z) != 0;
             npml += touch;
             list.push_back(make_int4(bx + (touch ? cgfd::kTilePml : 0), by, z.first, z.second));
           }
@@ -1501,7 +1525,7 @@ void make_tiles(cgfd_problem *p) {
       list.swap(ex);
       npml *= p->nshot;
     }
-    if (p->med != cgfd::MED_AC && p->src_bulk)
+    if (p->med != cgfd::MED_AC && p->src_tiles)
       for (int4 &e : list) {
         const int lo[3] = {(e.x & cgfd::kTileBxMask) * cgfd::TX, e.y * ty, e.z};
         const int hi[3] = {lo[0] + cgfd::TX - 1, lo[1] + ty - 1, e.w - 1};

@@ -348,7 +348,7 @@ __device__ __forceinline__ void bulk_tile(const StagePT<real_of<TC>> &p, const T
   }
   // sources inside the tile, after its stores (the last barrier orders them before these additions; the
   // RK combine is linear, so this equals adding to the right-hand side). A launch of its own after
-  // every stage took 3-4 us of the critical path (100x100x60: 259 -> 250 us per step)
+  // every stage takes 1-2 us of the critical path (64x64x64: 113 -> 107 us per step)
   if (tl.x & kTileSource)
     tile_sources(p, sp, shot, bx * TX, bx * TX + TX, by * TYT, by * TYT + TYT, kb, ke, tid, TX * TYT);
   if (bad) atomicOr(p.err, kErrWaveNonfinite);  // blow-up sentinel (drv_rk_curv_col.cu:507-510)

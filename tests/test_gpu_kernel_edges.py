@@ -8,10 +8,12 @@ equal to double rounding, so their read-back floats differ by one unit in the la
 import numpy as np
 import pytest
 
+import cgfd_b200
 from cgfd_b200 import Simulation, media_layer_gpu, CGFD_MEDIA_ARI, CGFD_MEDIA_HAR, CGFD_PREC_FP64
 from cgfd_b200.abi import Sources
 from cgfd_b200.formats import LayerModel
 from helpers import small_problem, random_wavefield
+from perf import cases
 
 pytestmark = pytest.mark.gpu
 
@@ -178,3 +180,83 @@ def test_fp64_batch_equals_its_shots_alone(medium):
             return [sim.wavefield(s) for s in range(sim.nshot)]
     for got, w in zip(run([p.src] * 3, waves), waves):
         np.testing.assert_array_equal(got, run(None, [w])[0])
+
+
+def _point_sources(p, at, amp=1.0):
+    n = len(at)
+    rng = np.random.default_rng(2)
+    cmp = amp * rng.uniform(-1, 1, (n, 9)).astype(np.float32) * np.array([1e12] * 3 + [1e16] * 6, np.float32)
+    coefs = np.zeros((n, 10), np.float32)
+    coefs[:, 0], coefs[:, 1] = 3.0, 0.02
+    return Sources(loc=np.array(at, np.float32), t_start=np.zeros(n, np.float32), wavelet=np.zeros(n, np.int32),
+                   wavelet_coefs=coefs, cmp=cmp, stf_length=6 * p.dt, cmp_type=3)
+
+
+INSIDE, CORNER = (40, 20, 14), (2, 2, 12)
+
+
+# shots' sources; launches of the source kernel a step (0: the tiles inject)
+@pytest.mark.parametrize("at,launches", [([[INSIDE]], 0), ([[INSIDE, (44, 22, 12)]], 4), ([[CORNER]], 4), ([[(40, 20, 25)]], 4),
+                                         ([[INSIDE], [(38, 14, 16)], [(44, 22, 9)]], 0), ([[INSIDE], [CORNER]], 4),
+                                         ([[INSIDE]] * 32, 0), ([[INSIDE]] * 33, 4)])
+def test_route_of_sources(at, launches):
+    p = small_problem("iso", 80, 41, 30, nsteps=2, npml=4, nsrc=0)
+    shots = [_point_sources(p, a) for a in at]
+    p.src = shots[0]
+    sim = Simulation(p, shots if len(shots) > 1 else None)
+    sim.set_timing(True)
+    sim.run(1)
+    assert sim.timing()["source"][1] == launches
+
+
+@pytest.mark.parametrize("precision", ["CGFD_PREC_FP32", "CGFD_PREC_U16_COEF", "CGFD_PREC_FP64"])
+@pytest.mark.parametrize("nshot", [1, 3])
+def test_tiles_inject_what_the_source_kernel_does(precision, nshot):
+    """A second source of zero moment sends a problem to the source kernel and adds nothing: bitwise."""
+    p = small_problem("iso", 80, 41, 30, nsteps=8, npml=4, nsrc=0, sta_grid=None)
+    p.precision = getattr(cgfd_b200, precision)
+    out = []
+    for more in (False, True):
+        shots = [_point_sources(p, [(40 + s, 20, 14 - s)]) for s in range(nshot)]
+        if more:
+            shots[-1] = _point_sources(p, [(39 + nshot, 20, 15 - nshot), (44, 22, 12)])
+            shots[-1].cmp[0] = _point_sources(p, [(40, 20, 14)]).cmp[0]
+            shots[-1].cmp[1] = 0
+        p.src = shots[0]
+        with Simulation(p, shots if nshot > 1 else None) as sim:
+            sim.run(8)  # the time function ends before the run does
+            out.append([sim.wavefield(s) for s in range(nshot)])
+            sim.set_timing(True)
+            sim.run(1)
+            assert sim.timing()["source"][1] == (4 if more else 0)
+    for a, b in zip(*out):
+        assert np.abs(b).max() > 0
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("shots", [0, 3])
+def test_tiles_inject_what_the_source_kernel_does_in_mixed_storage(shots):
+    """The same with FP16 stage levels, whose scale the injecting threads feed, from a wavefield and
+    sources of the tracked workloads (a source that starts at its full rate in a zero wavefield can
+    outgrow the scale's headroom within its first step, by either route)."""
+    c = cases._sim("run", "iso", 96, 80, 40, 16, 6, precision="mixed", shots=shots)
+    p, sources, waves = cases._inputs(c, 3)
+    sources = sources or [p.src]
+    out = []
+    for more in (False, True):
+        if more:
+            s = sources[-1]
+            sources[-1] = Sources(loc=np.concatenate([s.loc, s.loc + 2]), t_start=np.zeros(2, np.float32), wavelet=np.zeros(2, np.int32),
+                                  wavelet_coefs=np.repeat(s.wavelet_coefs, 2, 0), cmp=np.concatenate([s.cmp, 0 * s.cmp]),
+                                  stf_length=s.stf_length, cmp_type=s.cmp_type)
+        p.src = sources[0]
+        with Simulation(p, sources if shots else None) as sim:
+            for s, w in enumerate(waves):
+                sim.set_wavefield(w, s)
+            sim.run(15)
+            out.append([sim.wavefield(s) for s in range(sim.nshot)])
+            sim.set_timing(True)
+            sim.run(1)
+            assert sim.timing()["source"][1] == (4 if more else 0)
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
