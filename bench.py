@@ -323,7 +323,7 @@ def media_bench(local, steps=2000, media=("vti", "aniso", "ac", "vis")):
     cell-stage; acoustic: 16 wavefield + 11 coefficient accesses over every plane) per event-timed
     duration against the measured HBM peak. Each mode's problem is autotuned (tile shape, z chunk)
     before it runs. Last, the same grid with a visco-elastic medium (3 GMB mechanisms, FP32):
-    Gcell-stage/s and the event-timed stage (both passes) against its 593 B per cell-stage.
+    Gcell-stage/s and the event-timed stage against its 504 B per cell-stage.
     `media` picks the legs."""
     import torch
     from cgfd_b200 import (synth, Simulation, CGFD_PREC_FP32, CGFD_PREC_U16_COEF, CGFD_PREC_FP16_WAVE,
@@ -382,11 +382,11 @@ def media_bench(local, steps=2000, media=("vti", "aniso", "ac", "vis")):
             sim.close()
             out[f"{med}_{name}"] = rec
     # visco-elastic (GMB, 3 mechanisms; FP32 only, no FP64 build): the iso layers with Q, the
-    # same source and stations; the stage time covers the iso kernels in their right-hand-side
-    # mode and the attenuation pass. Bytes per cell-stage of this two-pass form, averaged over
-    # the 4 stages: the iso pass 30 floats (9 stage-input fields, 12 coefficients, 9 RHS) and the
-    # attenuation pass 118.25 (RHS, wave levels, 2 moduli, 6 weights and 18 memory variables per
-    # level touched: 98 / 143 / 143 / 89 floats at stages 0-3) = 593 B.
+    # same source and stations; the stage time covers the fused kernel of the bulk planes and the
+    # attenuation pass of the surface slab's 4. Bytes per cell-stage, averaged over the 4 stages: the
+    # fused kernel the iso stage's 48 floats (27 / 45 / 45 / 27 of the wave levels, 12 coefficients),
+    # 72 of the memory variables (18 per level touched: 54 / 90 / 90 / 54) and 6 weights = 504 B; the
+    # pass 118.25 floats (RHS, wave levels, 2 moduli, weights, memory variables: 98 / 143 / 143 / 89).
     if "vis" not in media:
         return out
     p = synth.make_problem(ni, nj, nk, 50.0, steps, dt=None, medium="vis", npml=20, nsrc=1, sta_grid=(10, 10),
@@ -406,14 +406,14 @@ def media_bench(local, steps=2000, media=("vti", "aniso", "ac", "vis")):
     sim.timing(reset=True)
     sim.enqueue(8)
     sim.synchronize()
-    bulk_ms, _ = sim.timing(reset=True)["bulk"]  # both passes of the 32 stages
+    bulk_ms, _ = sim.timing(reset=True)["bulk"]  # the 32 stages
     sim.set_timing(False)
     s = sim.seismograms()[:, :, :steps]
     zc = sim.zchunk
     sim.close()
-    bpc = 593.0
+    bpc = 504.0
     stage_ms = bulk_ms / 32
-    achieved = bpc * ni * nj * nk / (stage_ms * 1e-3) / 1e9
+    achieved = (bpc * (nk - 4) + 473.0 * 4) * ni * nj / (stage_ms * 1e-3) / 1e9
     out["vis_fp32"] = {"value": ni * nj * nk * 4 / (ms * 1e-3) / 1e9, "unit": UNIT, "ms_per_step": ms,
                        "nmaxwell": 3, "stage_ms": stage_ms, "bytes_per_cell_stage": bpc,
                        "roofline_frac": achieved / peak, "finite": bool(np.isfinite(s).all()), "zchunk": zc}
@@ -641,7 +641,7 @@ def main():
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak if achieved else None, "traffic": traffic, "traffic_capture": traffic_capture,
             "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)" if peak_kind == "measured" else "fallback",
-            "kernel": "k_stage_bulk_tma<iso> (interior-tile and PML-tile launches of one RK stage)",
+            "kernel": "k_stage_bulk_tma<iso> (one launch per RK stage)",
             "bytes_per_cell_stage": bpc, "cells_per_launch": bulk_cells,
             "kernel_ms": {k: (v[0] / v[1] if v[1] else None) for k, v in tim.items() if k != "launches"},
             "kernel_share": {k: (v[0] / ms_k if ms_k else None) for k, v in tim.items()
