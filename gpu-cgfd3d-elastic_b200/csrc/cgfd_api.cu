@@ -167,7 +167,7 @@ struct cgfd_problem {
   // d_wsc[18] from d_amax[2] (max |w| of velocity / stress) and d_srcb[nt_total][2] (largest
   // source increment of each step)
   int wave16 = 0;
-  // TMA bulk kernel tile lists for the current z chunk (interior tiles, then PML tiles)
+  // TMA stage kernels: tile lists of the current z chunk, by march direction (make_tiles)
   int4 *d_tiles = nullptr, *d_tiles_dn = nullptr;
   cgfd::BulkTiles tiles, tiles_dn;  // z layers upwards (backward z operators) / downwards
   // the flux pass and surface slab run on `side`, forked from and joined back into `stream`
@@ -1037,7 +1037,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
   p->wave16 = d->precision == CGFD_PREC_FP16_WAVE ? 1 : 0;
   p->fp64 = d->precision == CGFD_PREC_FP64 ? 1 : 0;
   p->esz = p->fp64 ? sizeof(double) : sizeof(float);
-  if (p->fp64 || p->vis) p->use_tma = false;  // the FP64 build runs the direct-load bulk kernel, visco-elastic media their own
+  if (p->fp64 || p->vis) p->use_tma = false;  // use_tma: the FP32 elastic kernel (tma64, vis_tma: theirs)
   p->vis_tma = p->vis && p->nmax <= cgfd::vis_bulk_max_mechanisms();
   p->device = d->device;
   CK(cudaSetDevice(p->device));
@@ -1143,6 +1143,7 @@ void build(cgfd_problem *p, const cgfd_problem_desc *d, int nshot, const cgfd_so
       p->jbuf[l] = dalloc_real(p, (size_t)6 * p->nmax * p->sf, B);
       CK(cudaMemsetAsync(p->jbuf[l], 0, sizeof(float) * 6 * p->nmax * p->sf, p->stream));
     }
+    // (every plane: the fused kernel leaves only the slab's to it, variant 0 all of them)
     p->d_rhs = dalloc_real(p, (size_t)9 * p->sf, B);
     CK(cudaMemsetAsync(p->d_rhs, 0, sizeof(float) * 9 * p->sf, p->stream));
     if (p->free_top) {
@@ -1459,7 +1460,7 @@ int default_chunk(const cgfd_problem *p) {
 // Tile lists of the TMA stage kernels: 32 x TY columns, split along z into chunks of about
 // nzc planes that never straddle a z-face boundary of the CFS-PML (so a column's faces are the same at
 // every plane of a tile). Entries (bx + flags + shot << 16, by, first plane, end plane): kTilePml on
-// tiles that a PML face box meets, kTileSource on those that hold sources.
+// tiles that a PML face box meets (acoustic), kTileSource on those that hold sources (elastic).
 // Order: strips of tile rows, each strip z layer by z layer, x fastest. A strip's layer holds
 // about as many blocks as the GPU keeps resident, so that a tile's x-y neighbours run beside it
 // at the same planes (their halo lines are read from DRAM once), and the tile's next chunk
@@ -1500,14 +1501,12 @@ void make_tiles(cgfd_problem *p) {
             }
   for (int dn = 0; dn < 2; dn++) {
     std::vector<int4> list;
-    int npml = 0;
     for (int s0 = 0; s0 < nby; s0 += strip)
       for (size_t zi = 0; zi < zr.size(); zi++) {
         const auto &z = zr[dn ? zr.size() - 1 - zi : zi];
         for (int by = s0; by < std::min(nby, s0 + strip); by++)
           for (int bx = 0; bx < nbx; bx++) {
-            const bool touch = face_axes(bx, by, z) != 0;
-            npml += touch;
+            const bool touch = p->med == cgfd::MED_AC && face_axes(bx, by, z) != 0;
             list.push_back(make_int4(bx + (touch ? cgfd::kTilePml : 0), by, z.first, z.second));
           }
       }
@@ -1523,7 +1522,6 @@ void make_tiles(cgfd_problem *p) {
           for (int sh = g0; sh < std::min(p->nshot, g0 + group); sh++)
             ex.push_back(make_int4(e.x + (sh << cgfd::kTileShotShift), e.y, e.z, e.w));
       list.swap(ex);
-      npml *= p->nshot;
     }
     if (p->med != cgfd::MED_AC && p->src_tiles)
       for (int4 &e : list) {
@@ -1545,7 +1543,6 @@ void make_tiles(cgfd_problem *p) {
     upload(p, dt, list.data(), list.size() * sizeof(int4));
     tl.list = dt;
     tl.n = (int)list.size();
-    tl.npml = npml;
   }
 }
 
@@ -2107,7 +2104,7 @@ int cgfd_autotune(cgfd_problem *p, int steps, int *chosen) {
     for (int c : {8, 10, 12, 14, 16, 20, 24, 32, 48, 64, 96, nbulk})
       if (c >= 1 && c <= nbulk && std::find(zc.begin(), zc.end(), c) == zc.end()) zc.push_back(c);
     // (tile shape, z chunk), the shapes interleaved so that a clock drifting during the tuning
-    // (power cap, temperature) does not favour one of them; the FP64 build has no TMA kernel
+    // (power cap, temperature) does not favour one of them; only the FP32 elastic kernel has two
     std::vector<std::pair<int, int>> cand;
     for (int c : zc)
       for (int sh = 0; sh < (p->use_tma ? 2 : 1); sh++) cand.emplace_back(sh, c);
@@ -2210,11 +2207,11 @@ int cgfd_set_bulk_variant(cgfd_problem *p, int tma) {
     return CGFD_ERR_UNSUPPORTED;
   }
   if (tma && p->fp64) {
-    set_err("the FP64 build runs the direct-load bulk kernel");
+    set_err("the FP64 build takes variant 0 only (direct loads; its own default kernel runs until then)");
     return CGFD_ERR_UNSUPPORTED;
   }
   if (tma && p->vis) {
-    set_err("visco-elastic media run the direct-load bulk kernel");
+    set_err("visco-elastic media take variant 0 only (direct loads; their own default kernel runs until then)");
     return CGFD_ERR_UNSUPPORTED;
   }
   if (p->med == cgfd::MED_AC) {  // acoustic: the TMA-pipelined (1) or direct-load (0) stage kernel

@@ -164,7 +164,7 @@ constexpr int kTileShotShift = 16, kTileShotMask = 0x7fff;  // bits 16-30: the s
 constexpr int kTileSource = INT_MIN;  // bit 31: smoothing points of the shot's sources lie in the tile
 struct BulkTiles {
   const int4 *list = nullptr;
-  int n = 0, npml = 0;  // entries, of which PML tiles
+  int n = 0;  // entries
 };
 // the TMA-pipelined acoustic stage (FP32; tm: the acoustic maps; 32 x TY tiles of every plane)
 int ac_tma_resident();
