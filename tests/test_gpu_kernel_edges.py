@@ -10,8 +10,9 @@ import pytest
 
 import cgfd_b200
 from cgfd_b200 import Simulation, media_layer_gpu, CGFD_MEDIA_ARI, CGFD_MEDIA_HAR, CGFD_PREC_FP64
-from cgfd_b200.abi import Sources
-from cgfd_b200.formats import LayerModel
+from cgfd_b200 import CGFD_MEDIA_LOC
+from cgfd_b200.abi import Sources, media_layer_any_gpu
+from cgfd_b200.formats import LayerMedia, LayerModel
 from helpers import small_problem, random_wavefield
 from perf import cases
 
@@ -260,3 +261,78 @@ def test_tiles_inject_what_the_source_kernel_does_in_mixed_storage(shots):
             assert sim.timing()["source"][1] == (4 if more else 0)
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("method", [CGFD_MEDIA_LOC, CGFD_MEDIA_HAR, CGFD_MEDIA_ARI])
+@pytest.mark.parametrize("medium", ["ac", "iso"])
+def test_layer_averages_with_gradients_and_powers(method, medium):
+    """Flat layers whose parameters rise with depth by powers 0, 1, 2 and between (dz^pow gradient in
+    double), on a Cartesian grid, isotropic and acoustic files, against the same sums in 64 bits. An
+    interface lies half a metre above a sub-point: the reference's integer test then takes the mean of
+    both layers. Tolerance: as above, 729 x 2^-24 of the sum, and a few roundings of the values."""
+    ni, nj, nk, dh = 9, 12, 17, 100.0
+    coord = np.zeros((3, nk + 6, nj + 6, ni + 6), np.float32)
+    coord[0] = (np.arange(-3, ni + 3) * dh)[None, None, :]
+    coord[1] = (np.arange(-3, nj + 3) * dh)[None, :, None]
+    coord[2] = (np.arange(-3, nk + 3) * dh - (nk - 1) * dh)[:, None, None]
+    tops = [float(coord[2].max()) + 500.0, -237.0, -612.0, -1099.5]
+    vals = {"rho": ([2500.0, 2600.0, 2700.0, 2900.0], [10.0, 0.02, 1e-5, 0.3], [0.0, 1.0, 2.0, 0.5]),
+            "vp": ([4000.0, 4800.0, 5500.0, 6500.0], [0.4, 1.0, 30.0, 1e-4], [0.5, 0.75, 0.0, 2.0]),
+            "vs": ([2300.0, 2700.0, 3200.0, 3750.0], [1e-4, 0.02, 0.3, 5.0], [2.0, 1.0, 0.5, 0.0])}
+    names = ("rho", "vp") if medium == "ac" else ("rho", "vp", "vs")
+    shape = (4, 4, 5)
+    flat = lambda v: np.array(v, np.float32)[:, None, None] * np.ones(shape, np.float32)  # noqa: E731
+    param = np.stack([np.stack([flat(v) for v in vals[n]]) for n in names])
+    m = LayerMedia(10 if medium == "ac" else 21, float(coord[0].min()) - 50, float(coord[1].min()) - 50, 1000.0, 1000.0,
+                   flat(tops), param)
+    got = media_layer_any_gpu(coord, m, 1 if medium == "ac" else 2, method)
+
+    def at(name, layer, dz):
+        v, g, p = (float(np.float32(q[layer])) for q in vals[name])
+        return v + dz ** p * g
+
+    def values(z):  # (rho, kappa) or (rho, lambda, mu) at elevation z
+        n = max(q for q in range(4) if tops[q] >= z)
+        layers = [n - 1, n] if n > 0 and int(tops[n] - z) == 0 else [n]
+        # (acoustic files: the layer above at the depth below the lower interface, as the reference does)
+        dz = {q: tops[n if medium == "ac" else q] - z for q in layers}
+        v = [np.mean([at(name, q, dz[q]) for q in layers]) for name in names]
+        if medium == "ac":
+            return np.array([v[0], v[0] * v[1] ** 2])
+        return np.array([v[0], v[0] * v[1] ** 2 - 2 * v[0] * v[2] ** 2, v[0] * v[2] ** 2])
+
+    mixed = 0
+    for k in range(1, nk + 5):
+        z = float(coord[2, k, 0, 0])
+        lo, hi = z - dh / 2, z + dh / 2
+        if method == CGFD_MEDIA_LOC or len({max(q for q in range(4) if tops[q] >= e) for e in (lo, hi)}) == 1:
+            want = values(z)
+        else:
+            mixed += 1
+            v = np.array([values(lo + (hi - lo) / 8 * s) for s in range(9)])
+            want = v.mean(0)
+            if method == CGFD_MEDIA_HAR and medium == "ac":
+                want[1] = 1 / np.mean(1 / v[:, 1])
+            elif method == CGFD_MEDIA_HAR:
+                mu = 1 / np.mean(1 / v[:, 2])
+                want = np.array([want[0], 1 / np.mean(1 / (v[:, 1] + 2 / 3 * v[:, 2])) - 2 / 3 * mu, mu])
+        np.testing.assert_allclose(got[:, k, 1:-1, 1:-1], want[:, None, None] * np.ones((len(want), nj + 4, ni + 4)),
+                                   rtol=5e-5, err_msg=f"plane {k}")
+    assert mixed == (0 if method == CGFD_MEDIA_LOC else 3)
+
+
+@pytest.mark.parametrize("nmax", [1, 3, 4, 5])
+@pytest.mark.parametrize("free", [True, False])
+def test_visco_against_64_bits(nmax, free):
+    """The attenuation of the fused kernel (up to 4 mechanisms) and of the separate pass against a
+    restatement in 64 bits that shares no code with them; 1e-5 x max |ref| per component and FP32 step."""
+    c = cases._sim("run", "vis", 70, 45, 37, 16, 6, free=free, nmax=nmax)
+    p, _, (wave,) = cases._inputs(c, 11)
+    ref = cases._Run64(c, p, p.src, wave)
+    with Simulation(p) as sim:
+        sim.set_wavefield(wave)
+        sim.run(5)
+        got = sim.wavefield()[:, 3:-3, 3:-3, 3:-3]
+    for it in range(5):
+        ref.step(it)
+    _close(got, ref.pre[:, 3:-3, 3:-3, 3:-3].cpu().numpy(), 5e-5)
